@@ -4,6 +4,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -12,6 +13,7 @@
 #include "bbts_b200.h"
 #include "common.h"
 #include "contraction.h"
+#include "f32tc.h"
 #include "gemm_f32.cuh"
 #include "gemm_tc.cuh"
 #include "stream_ops.cuh"
@@ -54,9 +56,16 @@ struct DeviceState {
   int sms = 148;
   uint32_t* status = nullptr;       // kernel status word
   uint32_t attr_done = 0;          // bitmask of tcgen05 kernels with smem attribute set
+  cudaMemPool_t scratch = nullptr;  // scratch_alloc
 };
 static std::mutex g_dev_mu;
 static DeviceState g_dev[64];
+// Scratch kept by the pool across synchronisations. The device's default pool
+// keeps none: a call after a synchronisation then maps its scratch again, which
+// took 3-4 ms (a 201 x 160 x 130 contraction 4.0 ms alone against 0.15 ms among others).
+// 512 MiB holds the operand planes of an 8192^2 by 8192 x 2048 f32 product; the
+// runtime takes it back (scratch_trim) before it reports the device out of memory.
+constexpr uint64_t kScratchKeep = 512ull << 20;
 
 template <int BN, bool AMN, bool BMN, bool FP8, bool EP8 = false>
 static int set_tc_attr() {
@@ -118,6 +127,7 @@ static int init_tc_attributes() {
                  (const void*)k_stream_bulk_inline<false>, (const void*)k_stream_bulk_inline<true>})
     rc |= cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kBulkSmemMax) != cudaSuccess;
   rc |= gather_bulk_init() != BBX_OK;
+  rc |= f3_init() != BBX_OK;
   return rc ? BBX_ERR_CUDA : BBX_OK;
 }
 
@@ -136,6 +146,16 @@ int device_state(DeviceState** out) {
     // inside a stream capture.
     int rc = init_tc_attributes();
     if (rc) return rc;
+    if (!d.scratch) {
+      cudaMemPoolProps props;
+      memset(&props, 0, sizeof(props));
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      BBX_CUDA(cudaMemPoolCreate(&d.scratch, &props));
+      uint64_t keep = kScratchKeep;
+      BBX_CUDA(cudaMemPoolSetAttribute(d.scratch, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
     d.attr_done = 0xFFFFFFFFu;
     d.ready = true;
   }
@@ -150,6 +170,31 @@ int device_status_and_sms(uint32_t** status, int* sms) {
   *status = d->status;
   *sms = d->sms;
   return BBX_OK;
+}
+
+// The pool is thread-safe and orders a block's reuse by stream.
+void* scratch_alloc(size_t bytes, void* stream) {
+  DeviceState* d;
+  if (device_state(&d)) return nullptr;
+  void* p = nullptr;
+  const cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, d->scratch, (cudaStream_t)stream);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // a failed allocation must not show up at the next launch check
+    set_error(BBX_ERR_CUDA, "scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
+    return nullptr;
+  }
+  return p;
+}
+
+void scratch_free(void* p, void* stream) {
+  if (p) cudaFreeAsync(p, (cudaStream_t)stream);
+}
+
+void scratch_trim() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  std::lock_guard<std::mutex> lk(g_dev_mu);
+  if (g_dev[dev].scratch) cudaMemPoolTrimTo(g_dev[dev].scratch, 0);
 }
 
 static inline int grid_for(long long work_items, int threads, int sms) {
@@ -186,7 +231,7 @@ static int get_encode_fn(EncodeTiledFn* fn) {
 // `ld` elements; box = box_cols x box_rows, 128-byte swizzle, zero OOB fill.
 static int make_map(CUtensorMap* map, const void* base, int dtype, long long rows, long long cols,
                     long long ld, int box_cols, int box_rows, bool swizzle = true) {
-  EncodeTiledFn enc;
+  EncodeTiledFn enc = nullptr;
   int rc = get_encode_fn(&enc);
   if (rc) return rc;
   const int esz = dtype == BBX_E4M3 ? 1 : dtype == BBX_F32 ? 4 : 2;
@@ -204,6 +249,24 @@ static int make_map(CUtensorMap* map, const void* base, int dtype, long long row
     return set_error(BBX_ERR_INVALID,
                      "cuTensorMapEncodeTiled failed (%d): rows=%lld cols=%lld ld=%lld box=%dx%d",
                      (int)r, rows, cols, ld, box_cols, box_rows);
+  return BBX_OK;
+}
+
+int make_map3(void* map, const void* base, long long cols, long long rows, long long z, long long pitch,
+              long long z_stride, int box_cols, int box_rows) {
+  EncodeTiledFn enc = nullptr;
+  int rc = get_encode_fn(&enc);
+  if (rc) return rc;
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)z};
+  cuuint64_t strides[2] = {(cuuint64_t)(pitch * 2), (cuuint64_t)(z_stride * 2)};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc((CUtensorMap*)map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
+                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return set_error(BBX_ERR_INVALID, "cuTensorMapEncodeTiled failed (%d): rows=%lld cols=%lld z=%lld pitch=%lld", (int)r,
+                     rows, cols, z, pitch);
   return BBX_OK;
 }
 
@@ -239,6 +302,14 @@ static int launch_tc(int bn, bool amn, bool bmn, bool fp8, bool ep8, const TcArg
   TC_CASE(128, true, false, true) TC_CASE(128, true, true, true)
 #undef TC_CASE
   return set_error(BBX_ERR_UNSUPPORTED, "no tcgen05 variant for tile_n=%d", bn);
+}
+
+template <typename Args>
+static void launch_f32_v(bool ta, bool tb, dim3 grid, cudaStream_t st, const Args& args) {
+  if (!ta && !tb) k_gemm_f32_v<false, false><<<grid, 256, 0, st>>>(args);
+  else if (!ta) k_gemm_f32_v<false, true><<<grid, 256, 0, st>>>(args);
+  else if (!tb) k_gemm_f32_v<true, false><<<grid, 256, 0, st>>>(args);
+  else k_gemm_f32_v<true, true><<<grid, 256, 0, st>>>(args);
 }
 
 // Validates one public problem and fills the device record (minus tile_start).
@@ -419,11 +490,35 @@ int bbx_matmul_f32(const float* a, const float* b, float* c, int m, int n, int k
   dim3 grid((n + F32_BN - 1) / F32_BN, (m + F32_BM - 1) / F32_BM, batch);
   if (grid.y > 65535) return set_error(BBX_ERR_INVALID, "m too large");
   cudaStream_t st = (cudaStream_t)stream;
+  // On the tensor cores where f3_wanted says so. Not inside a stream capture:
+  // the operand planes are stream-ordered scratch, and an allocation node would
+  // restrict what the caller may do with the captured graph. Without room for the
+  // planes the SIMT kernel, which needs none, runs. A fused ReLU marks a
+  // pre-activation (FmaChain).
+  if (!relu && !FmaChain::active() && f3_wanted(m, n, k, batch)) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    BBX_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap == cudaStreamCaptureStatusNone) {
+      F3Mat mats[2] = {trans_a ? f3_dense(a, k, m, lda, batch, stride_a, true) : f3_dense(a, m, k, lda, batch, stride_a, false),
+                       trans_b ? f3_dense(b, n, k, ldb, batch, stride_b, false) : f3_dense(b, k, n, ldb, batch, stride_b, true)};
+      const size_t ba = f3_mat_bytes(mats[0]), bb = f3_mat_bytes(mats[1]);
+      if (void* ws = scratch_alloc(ba + bb, stream)) {
+        mats[0].ws = ws;
+        mats[1].ws = (char*)ws + ba;
+        F3Spec s;
+        s.a = 0; s.b = 1;
+        s.c = c; s.bias = bias;
+        s.m = m; s.n = n; s.k = k;
+        s.ldc = ldc; s.c_batch = stride_c;
+        s.alpha = alpha; s.beta = beta; s.relu = relu;
+        const int rc = f3_run(mats, s, stream);
+        scratch_free(ws, stream);
+        return rc;
+      }
+    }
+  }
   if (f32_gemm_vector_ok(g)) {
-    if (!trans_a && !trans_b) k_gemm_f32_v<false, false><<<grid, 256, 0, st>>>(g);
-    else if (!trans_a) k_gemm_f32_v<false, true><<<grid, 256, 0, st>>>(g);
-    else if (!trans_b) k_gemm_f32_v<true, false><<<grid, 256, 0, st>>>(g);
-    else k_gemm_f32_v<true, true><<<grid, 256, 0, st>>>(g);
+    launch_f32_v(trans_a != 0, trans_b != 0, grid, st, g);
     BBX_CHECK_LAUNCH("k_gemm_f32_v");
     return BBX_OK;
   }
@@ -431,6 +526,76 @@ int bbx_matmul_f32(const float* a, const float* b, float* c, int m, int n, int k
   BBX_CHECK_LAUNCH("k_gemm_f32");
   return BBX_OK;
 }
+
+}  // extern "C"
+
+namespace bbx {
+struct F32SimtPlan {
+  struct Part { int mode, tiles; F32GroupArgs args; };
+  std::vector<Part> parts;  // one launch each
+};
+
+int f32_simt_plan_create(const F32SimtSpec* specs, int n, F32SimtPlan** out) {
+  if (!specs || n <= 0 || !out) return set_error(BBX_ERR_INVALID, "bad f32 group arguments");
+  std::vector<F32GemmArgs> gs(n);
+  std::vector<std::pair<int, int>> order;  // (kernel, index), the longest K first within a kernel
+  for (int i = 0; i < n; ++i) {
+    const F32SimtSpec& q = specs[i];
+    if (!q.a || !q.b || !q.c || q.m <= 0 || q.n <= 0 || q.k < 0)
+      return set_error(BBX_ERR_INVALID, "f32 group: product %d: m=%d n=%d k=%d", i, q.m, q.n, q.k);
+    F32GemmArgs& g = gs[i];
+    memset(&g, 0, sizeof(g));
+    g.a = q.a; g.b = q.b; g.c = q.c;
+    g.m = q.m; g.n = q.n; g.k = q.k;
+    g.lda = q.lda; g.ldb = q.ldb; g.ldc = q.ldc;
+    g.trans_a = q.trans_a; g.trans_b = q.trans_b;
+    g.alpha = 1.f;
+    order.push_back({f32_gemm_vector_ok(g) ? 1 + 2 * (q.trans_a != 0) + (q.trans_b != 0) : 0, i});
+  }
+  std::stable_sort(order.begin(), order.end(), [&](const auto& x, const auto& y) {
+    return x.first != y.first ? x.first < y.first : specs[x.second].k > specs[y.second].k;
+  });
+  auto p = std::make_unique<F32SimtPlan>();
+  for (const auto& o : order) {
+    const F32GemmArgs& g = gs[o.second];
+    const int tn = (g.n + F32_BN - 1) / F32_BN;
+    const long long tiles = (long long)tn * ((g.m + F32_BM - 1) / F32_BM);
+    if (tiles > (1ll << 30)) return set_error(BBX_ERR_INVALID, "f32 group: too many tiles");
+    if (p->parts.empty() || p->parts.back().mode != o.first || p->parts.back().args.count == kF32GroupMax ||
+        p->parts.back().tiles + tiles > (1ll << 30)) {
+      p->parts.emplace_back();
+      memset(&p->parts.back(), 0, sizeof(F32SimtPlan::Part));
+      p->parts.back().mode = o.first;
+    }
+    F32SimtPlan::Part& q = p->parts.back();
+    const int i = q.args.count++;
+    q.args.g[i] = g;
+    q.args.tile_start[i] = q.tiles;
+    q.args.tiles_n[i] = tn;
+    q.tiles += (int)tiles;
+  }
+  *out = p.release();
+  return BBX_OK;
+}
+
+int f32_simt_plan_launch(F32SimtPlan* p, void* stream) {
+  if (!p) return set_error(BBX_ERR_INVALID, "null f32 group");
+  cudaStream_t st = (cudaStream_t)stream;
+  for (const auto& q : p->parts) {
+    const F32GemmArgs& g = q.args.g[0];
+    if (q.args.count == 1 && q.mode != 0)  // the single-product form: see k_gemm_f32_v
+      launch_f32_v(g.trans_a != 0, g.trans_b != 0, dim3((g.n + F32_BN - 1) / F32_BN, (g.m + F32_BM - 1) / F32_BM), st, g);
+    else if (q.mode == 0) k_gemm_f32<<<q.tiles, 256, 0, st>>>(q.args);
+    else launch_f32_v(((q.mode - 1) & 2) != 0, ((q.mode - 1) & 1) != 0, dim3(q.tiles), st, q.args);
+    BBX_CHECK_LAUNCH("k_gemm_f32 group");
+  }
+  return BBX_OK;
+}
+
+void f32_simt_plan_destroy(F32SimtPlan* p) { delete p; }
+}  // namespace bbx
+
+extern "C" {
 
 int bbx_tc_plan_create(int in_dtype, const bbx_tc_problem_t* problems, int count, int tile_n,
                        bbx_tc_plan_t** out) {
@@ -665,8 +830,8 @@ int bbx_quantize_e4m3(int src_dtype, const void* in, void* out, int rows, int co
   cudaStream_t st = (cudaStream_t)stream;
   // the absmax word is stream-ordered scratch of this call, so quantisations
   // on different streams never share it
-  unsigned int* amax = nullptr;
-  BBX_CUDA(cudaMallocAsync((void**)&amax, 4, st));
+  unsigned int* amax = (unsigned int*)scratch_alloc(4, st);
+  if (!amax) return BBX_ERR_CUDA;
   BBX_CUDA(cudaMemsetAsync(amax, 0, 4, st));
   uint8_t* o = (uint8_t*)out;
   cudaError_t le;
@@ -677,7 +842,7 @@ int bbx_quantize_e4m3(int src_dtype, const void* in, void* out, int rows, int co
     const __nv_bfloat16* i = (const __nv_bfloat16*)in;
     le = launch_quantize_batch(&i, &o, 1, rows, cols, transpose, amax, scale_out, d->sms, st);
   }
-  cudaFreeAsync(amax, st);
+  scratch_free(amax, st);
   if (le != cudaSuccess) return set_error(BBX_ERR_CUDA, "quantize_e4m3: %s", cudaGetErrorString(le));
   return BBX_OK;
 }
@@ -695,15 +860,15 @@ int bbx_quantize_e4m3_batched(int src_dtype, const void* const* in, void* const*
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   // one absmax word per block, stream-ordered scratch of this call
-  unsigned int* amax = nullptr;
-  BBX_CUDA(cudaMallocAsync((void**)&amax, sizeof(unsigned int) * count, st));
+  unsigned int* amax = (unsigned int*)scratch_alloc(sizeof(unsigned int) * count, st);
+  if (!amax) return BBX_ERR_CUDA;
   BBX_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned int) * count, st));
   cudaError_t le = src_dtype == BBX_F32
                        ? launch_quantize_batch((const float* const*)in, (uint8_t* const*)out, count, rows, cols,
                                                transpose, amax, scales_out, d->sms, st)
                        : launch_quantize_batch((const __nv_bfloat16* const*)in, (uint8_t* const*)out, count, rows,
                                                cols, transpose, amax, scales_out, d->sms, st);
-  cudaFreeAsync(amax, st);
+  scratch_free(amax, st);
   if (le != cudaSuccess) return set_error(BBX_ERR_CUDA, "quantize_e4m3_batched: %s", cudaGetErrorString(le));
   return BBX_OK;
 }

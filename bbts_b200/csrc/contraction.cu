@@ -25,6 +25,7 @@
 #include "bbts_b200.h"
 #include "common.h"
 #include "contraction.h"
+#include "f32tc.h"
 #include "ptx.cuh"
 
 namespace bbx {
@@ -659,32 +660,52 @@ extern "C" int bbx_contraction(const float* lhs, int rank_l, const long long* di
     return set_error(BBX_ERR_UNSUPPORTED, "contraction precision %d", precision);
   const bool bf16 = precision == BBX_BF16;
   ContractionLowering L;
-  int rc = lower_contraction(rank_l, dims_l, modes_l, rank_r, dims_r, modes_r, rank_o, modes_o, bf16, &L);
+  // lowered for the tensor cores first: its group sizes decide where an f32 contraction runs
+  int rc = lower_contraction(rank_l, dims_l, modes_l, rank_r, dims_r, modes_r, rank_o, modes_o, true, &L);
   if (rc) return rc;
   if (L.empty) return BBX_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  // one scratch block: the staged operands, then Ct where the output needs a last gather
+  auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t cbytes = L.direct ? 0 : (size_t)(L.nb * L.nn * L.nm * 4);
   const int esz = bf16 ? 2 : 4;
-  void *Lc = nullptr, *Rc = nullptr;
-  float* Ct = nullptr;
-  cudaError_t e;
-  e = cudaMallocAsync(&Lc, (size_t)(L.lc_elems * esz + 16), st);
-  if (e != cudaSuccess) return set_error(BBX_ERR_CUDA, "cudaMallocAsync: %s", cudaGetErrorString(e));
-  e = cudaMallocAsync(&Rc, (size_t)(L.rc_elems * esz + 16), st);
-  if (e != cudaSuccess) { cudaFreeAsync(Lc, st); return set_error(BBX_ERR_CUDA, "cudaMallocAsync: %s", cudaGetErrorString(e)); }
-  if (!L.direct) {
-    e = cudaMallocAsync((void**)&Ct, (size_t)(L.nb * L.nn * L.nm * 4), st);
-    if (e != cudaSuccess) { cudaFreeAsync(Lc, st); cudaFreeAsync(Rc, st); return set_error(BBX_ERR_CUDA, "cudaMallocAsync: %s", cudaGetErrorString(e)); }
+  F3Mat mats[2];
+  F3Spec spec;
+  size_t lbytes = 0, rbytes = 0;
+  char* ws = nullptr;
+  bool f3 = !bf16 && !FmaChain::active() && f3_contraction_wanted(L);
+  if (f3) {
+    f3_contraction(L, lhs, rhs, nullptr, alpha, &mats[0], &mats[1], &spec);
+    lbytes = f3_mat_bytes(mats[0]);
+    rbytes = f3_mat_bytes(mats[1]);
+    ws = (char*)scratch_alloc(up(lbytes) + up(rbytes) + cbytes, stream);
+    f3 = ws != nullptr;  // the planes take half as much again as the f32 staging below
   }
-  float* C = L.direct ? out : Ct;
-  rc = launch_gather(lhs, Lc, bf16, L.ga, L.nl, st);
-  if (!rc) rc = launch_gather(rhs, Rc, bf16, L.gb, L.nr, st);
-  if (!rc) {
-    const long long pitch = L.pk;
+  if (!f3) {
     if (!bf16) {
-      rc = bbx_matmul_f32((const float*)Rc, (const float*)Lc, C, (int)L.nn, (int)L.nm, (int)L.kdim, pitch,
-                          pitch, L.nm, 0, 1, alpha, 0.f, nullptr, 0, (int)L.nb, L.nn * pitch, L.nm * pitch,
-                          L.nn * L.nm, stream);
-    } else {
+      rc = lower_contraction(rank_l, dims_l, modes_l, rank_r, dims_r, modes_r, rank_o, modes_o, false, &L);
+      if (rc) return rc;
+    }
+    lbytes = (size_t)(L.lc_elems * esz + 16);
+    rbytes = (size_t)(L.rc_elems * esz + 16);
+    ws = (char*)scratch_alloc(up(lbytes) + up(rbytes) + cbytes, stream);
+    if (!ws) return BBX_ERR_CUDA;
+  }
+  void *Lc = ws, *Rc = ws + up(lbytes);
+  float* Ct = L.direct ? nullptr : (float*)(ws + up(lbytes) + up(rbytes));
+  float* C = L.direct ? out : Ct;
+  if (f3) {
+    mats[0].ws = Lc;
+    mats[1].ws = Rc;
+    spec.c = C;
+    rc = f3_run(mats, spec, stream);
+  } else {
+    rc = launch_gather(lhs, Lc, bf16, L.ga, L.nl, st);
+    if (!rc) rc = launch_gather(rhs, Rc, bf16, L.gb, L.nr, st);
+    if (!rc && !bf16) {
+      rc = bbx_matmul_f32((const float*)Rc, (const float*)Lc, C, (int)L.nn, (int)L.nm, (int)L.kdim, L.pk, L.pk, L.nm, 0, 1,
+                          alpha, 0.f, nullptr, 0, (int)L.nb, L.nn * L.pk, L.nm * L.pk, L.nn * L.nm, stream);
+    } else if (!rc) {
       std::vector<bbx_tc_problem_t> probs((size_t)L.nb);
       for (long long b = 0; b < L.nb; ++b) {
         bbx_tc_problem_t& q = probs[(size_t)b];
@@ -701,8 +722,6 @@ extern "C" int bbx_contraction(const float* lhs, int rank_l, const long long* di
     }
   }
   if (!rc && !L.direct) rc = launch_gather(Ct, out, false, L.go, L.no, st);
-  cudaFreeAsync(Lc, st);
-  cudaFreeAsync(Rc, st);
-  if (Ct) cudaFreeAsync(Ct, st);
+  scratch_free(ws, stream);
   return rc;
 }

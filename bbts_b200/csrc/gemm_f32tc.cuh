@@ -1,0 +1,717 @@
+// FP32 block matmul on the tensor cores.
+//
+// An f32 value is the exact sum of three bf16 values (8 significant bits each):
+//     a = a0 + 2^-8 a1 + 2^-16 a2,   a0 = bf16(a), a1 = bf16((a - a0) 2^8), ...
+// The planes are scaled so that each has a0's exponent range: no plane
+// underflows before a itself does. A product a b is then
+//     a0 b0 + 2^-8 (a0 b1 + a1 b0) + 2^-16 (a0 b2 + a1 b1 + a2 b0) + O(2^-26 |a b|),
+// six bf16 products that tcgen05.mma forms exactly and accumulates in f32. The
+// three dropped products are below a quarter of an ulp of a b.
+//
+// Accumulation. The tensor core truncates when it accumulates, so a long K loop
+// in one accumulator loses about K * 2^-26 (relative, measured: 1.0e-6 at K = 1024, 4.0e-6
+// at K = 4096, where the FMA chain of k_gemm_f32 loses 5.7e-7 and 1.2e-6). Here
+// the MMA accumulates only kF3BK = 64 steps of K: the 2^-16 products first, then the
+// accumulator is scaled by 2^-8 in the MMA itself (scale-input-d) and takes the
+// 2^-8 products, then once more and the leading product, so only the last four
+// MMAs truncate at the size of the result. The epilogue warps add each chunk to
+// FP32 registers with round-to-nearest while the next chunk runs in the other
+// TMEM buffer.
+//
+// Operands are read from their split planes (k_f32_split): TMA tiles of one
+// plane through a 3-D map (columns, rows, plane * batch + b), in whichever
+// major-ness the block has. A stage holds the six plane tiles of a chunk (128
+// rows x 64 of K, 16 KiB each), two stages fill the shared memory, and each tile is
+// handed back on its own as soon as the last product that reads it retires.
+//
+// Shapes: PAIR, a 256 x 256 tile on two SMs (cta_group::2: each SM loads 128
+// rows of A and of B), and a 128 x 128 tile on one SM for groups with too few tiles to
+// fill the chip with pairs. Both compute each output by the same chain of
+// operations, so the shape changes no bit of the result. Shared memory sets the pace of
+// the smaller: per chunk of K its MMAs read 24 x 8 KiB and the TMA writes 96 KiB at
+// 128 bytes a cycle, 2300 cycles where the tensor pipe needs 1536 (measured 2190); the pair
+// spreads the same traffic over the 3072 cycles of a tile twice as wide (measured 3600;
+// a 256 x 128 pair measured 2950, more per output than either).
+//
+// The producer and MMA warps run converged, with one elected lane issuing, so that
+// the TMA and MMA operands are uniform; a problem's fields are read once per tile
+// into registers, from the kernel parameters when there is a single problem.
+//
+// A problem whose operands could leave the range of the scheme (non-finite, or
+// large enough that a partial sum could overflow where an FP32 FMA chain does
+// not; see f3_in_range) is computed by the epilogue threads with FP32 FMAs in K
+// order, as k_gemm_f32 does.
+#pragma once
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include "ptx.cuh"
+#include "tile_order.h"
+
+namespace bbx {
+
+constexpr int kF3BK = 64;
+constexpr int kF3Tile = 128 * kF3BK * 2;      // one plane tile of 128 rows, 16 KiB
+constexpr int kF3Stage = 6 * kF3Tile;         // A0 A1 A2 B0 B1 B2
+constexpr int kF3MaxProblems = 256;           // per launch
+constexpr int kF3EpiPitch = 20;               // floats; 80-byte rows keep 16-byte accesses conflict-free
+constexpr int kF3EpiSlot = 32 * kF3EpiPitch * 4;
+constexpr int kF3EpiWarps = 8;
+constexpr int kF3Threads = 64 + 32 * kF3EpiWarps;
+constexpr int kF3Smem =
+    2 * kF3Stage + 1024 /* align slack */ + kF3EpiWarps * kF3EpiSlot + 256 /* barriers */ + kF3MaxProblems * 16;
+static_assert(kF3Smem <= 232448, "dynamic shared memory per CTA");
+
+// One (batched) product. 64-byte alignment is required by the tensor maps.
+struct F3Fields {
+  const __nv_bfloat16* a;      // plane 0 of the operands, for problems out of range
+  const __nv_bfloat16* b;
+  float* c;
+  const float* bias;
+  const uint32_t* amax_a;      // na / nb partial maxima of |a| and |b| (float bits), written by the split
+  const uint32_t* amax_b;
+  // element (row, k) of A's plane p: a + p * a_plane + batch * a_batch + row * a_row + k * a_k, and so on
+  long long a_plane, a_row, a_k, a_batch, b_plane, b_col, b_k, b_batch, ldc, c_batch;
+  int m, n, k, batch;
+  int na, nb;
+  int tile_start, tiles_m, tiles_n;
+  int a_mn, b_mn;              // operand tiles are MN-major
+  int c_col;                   // element (i, j) of C at c[i + j * ldc], else c[i * ldc + j]
+  float alpha, beta;
+  int relu;
+};
+struct alignas(64) F3Problem {
+  CUtensorMap tmap_a, tmap_b;  // split planes, box 64 columns x 128 rows (K-major) or 64 x 64 (MN-major)
+  F3Fields f;
+};
+
+struct F3Args {
+  const F3Problem* table;  // device table, or nullptr: `one`
+  int num_problems;
+  int total_tiles;
+  uint32_t* status;
+  F3Problem one;
+};
+
+// |a| < 2^ea, |b| < 2^eb for the maxima's exponents. The largest partial sum of
+// the scheme is below 3 K 2^(ea + eb) < 2^(ea + eb + lk + 2): kept below 2^127, so nothing
+// overflows that an FMA chain would not. The upper limit on each operand keeps
+// bf16(a) finite. Products that are all below 2^-80 are left to the FMA chain,
+// which rounds them to f32 subnormals as the reference does.
+__host__ __device__ __forceinline__ bool f3_in_range(uint32_t amax, uint32_t bmax, int k) {
+  if (amax >= 0x7F7F8000u || bmax >= 0x7F7F8000u) return false;  // also inf and NaN
+  if (amax == 0 || bmax == 0) return true;
+  const int ea = (int)(amax >> 23) - 126, eb = (int)(bmax >> 23) - 126;
+#ifdef __CUDA_ARCH__
+  const int lk = 32 - __clz(k - 1);  // 2^lk >= k
+#else
+  int lk = 0;
+  while ((1ll << lk) < k) ++lk;
+#endif
+  return ea + eb + lk + 2 <= 127 && ea + eb >= -80;
+}
+
+// ------------------------------------------------------------------ split into planes
+// One matrix (or gathered tensor) to split: rows indexed by up to three outer
+// dimensions, `len` elements along a row.
+struct F3Split {
+  const float* src;
+  __nv_bfloat16* dst;          // plane p at dst + p * plane
+  long long plane;             // elements
+  long long odims[3], istride[3], ostride[3];  // outer dims, outermost first; unused ones have extent 1
+  long long len, inner, oinner;  // elements of a row, their source and destination strides
+  long long items;             // rows * ceil(len / 8)
+  long long items_per_chunk;
+  uint32_t* amax;              // one word per chunk
+  int chunk_start;             // first chunk of this record in the launch
+  int rank_s;                  // modes summed at each element (0: none)
+  long long sdims[4], sstride[4];
+};
+
+struct F3SplitArgs {
+  const F3Split* table;        // device table, or nullptr: `inl`
+  int count;
+  F3Split inl[2];
+};
+
+// bf16 of a finite value, rounded to nearest, but never to infinity.
+__device__ __forceinline__ __nv_bfloat16 f3_bf16_finite(float x) {
+  const __nv_bfloat16 p = __float2bfloat16_rn(x);
+  return fabsf(__bfloat162float(p)) <= 3.3895314e38f ? p : __ushort_as_bfloat16((unsigned short)(__float_as_uint(x) >> 16));
+}
+
+// The planes of any f32 value: f3_join gives the value back exactly (a NaN as a NaN).
+__device__ __forceinline__ void f3_split1(float x, __nv_bfloat16& p0, __nv_bfloat16& p1, __nv_bfloat16& p2) {
+  const uint32_t mag = __float_as_uint(x) & 0x7FFFFFFFu;
+  if (mag >= 0x7F800000u) {
+    p0 = __float2bfloat16_rn(x);
+    p1 = p2 = __ushort_as_bfloat16(0);
+    return;
+  }
+  p0 = mag < 0x7F000000u ? __float2bfloat16_rn(x) : f3_bf16_finite(x);
+  const float r1 = __fmul_rn(__fsub_rn(x, __bfloat162float(p0)), 256.f);  // exact
+  p1 = mag < 0x7F000000u ? __float2bfloat16_rn(r1) : f3_bf16_finite(r1);
+  p2 = __float2bfloat16_rn(__fmul_rn(__fsub_rn(r1, __bfloat162float(p1)), 256.f));
+}
+
+__device__ __forceinline__ float f3_join(const __nv_bfloat16* p, long long plane) {
+  const float lo = __fadd_rn(__fmul_rn(__bfloat162float(p[plane]), 1.f / 256.f),
+                             __fmul_rn(__bfloat162float(p[2 * plane]), 1.f / 65536.f));
+  return __fadd_rn(__bfloat162float(p[0]), lo);
+}
+
+// Chunk blockIdx.x of the launch: its record's items [i0, i1), eight elements
+// of one row each. 4 bytes read and 6 written per element: HBM-bound; 16-byte
+// loads where the row starts on a 16-byte boundary, 16-byte stores of the planes
+// where the row of the planes does. Each CTA writes the maximum of |x| over its
+// chunk as one word, so no counter has to be cleared before the launch.
+__global__ void __launch_bounds__(256) k_f32_split(const __grid_constant__ F3SplitArgs args) {
+  const int chunk = blockIdx.x;
+  int lo = 0, hi = args.count - 1;
+  const F3Split* const recs = args.table ? args.table : args.inl;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (recs[mid].chunk_start <= chunk) lo = mid; else hi = mid - 1;
+  }
+  const F3Split& r = recs[lo];
+  const float* __restrict__ src = r.src;
+  __nv_bfloat16* const dst = r.dst;
+  const long long plane = r.plane, len = r.len, inner = r.inner;
+  const long long per_row = (len + 7) >> 3;
+  const long long i0 = (chunk - r.chunk_start) * r.items_per_chunk;
+  const long long i1 = min(i0 + r.items_per_chunk, r.items);
+  const long long od1 = r.odims[1], od2 = r.odims[2];
+  const long long is0 = r.istride[0], is1 = r.istride[1], is2 = r.istride[2];
+  const long long os0 = r.ostride[0], os1 = r.ostride[1], os2 = r.ostride[2];
+  const bool small = r.items < (1ll << 31) && od1 * od2 < (1ll << 31);
+  uint32_t mx = 0;
+  for (long long it = i0 + threadIdx.x; it < i1; it += blockDim.x) {
+    long long row, c8;
+    if (small) {  // 32-bit division
+      row = (uint32_t)it / (uint32_t)per_row;
+      c8 = it - row * per_row;
+    } else {
+      row = it / per_row;
+      c8 = it - row * per_row;
+    }
+    long long q, d2, d1;
+    if (small) {
+      q = (uint32_t)row / (uint32_t)od2;
+      d2 = row - q * od2;
+      const long long q1 = (uint32_t)q / (uint32_t)od1;
+      d1 = q - q1 * od1;
+      q = q1;
+    } else {
+      q = row / od2;
+      d2 = row - q * od2;
+      const long long q1 = q / od1;
+      d1 = q - q1 * od1;
+      q = q1;
+    }
+    const long long e = c8 * 8;
+    const int cnt = (int)min(8ll, len - e);
+    const float* sp = src + q * is0 + d1 * is1 + d2 * is2 + e * inner;
+    float v[8];
+    if (r.rank_s > 0) {
+      long long ns = 1;
+      for (int d = 0; d < r.rank_s; ++d) ns *= r.sdims[d];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        v[u] = 0.f;
+        if (u < cnt)
+          for (long long s = 0; s < ns; ++s) {
+            long long rem = s, off = 0;
+            for (int d = 0; d < r.rank_s; ++d) {
+              off += (rem % r.sdims[d]) * r.sstride[d];
+              rem /= r.sdims[d];
+            }
+            v[u] += sp[u * inner + off];
+          }
+      }
+    } else if (cnt == 8 && inner == 1 && (((uintptr_t)sp) & 15) == 0) {
+      const float4 a = __ldg((const float4*)sp), b = __ldg((const float4*)sp + 1);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+      v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = u < cnt ? __ldg(sp + u * inner) : 0.f;
+    }
+    uint32_t p[3][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      __nv_bfloat16 x[3], y[3];
+      mx = max(mx, max(__float_as_uint(v[2 * u]) & 0x7FFFFFFFu, __float_as_uint(v[2 * u + 1]) & 0x7FFFFFFFu));
+      f3_split1(v[2 * u], x[0], x[1], x[2]);
+      f3_split1(v[2 * u + 1], y[0], y[1], y[2]);
+#pragma unroll
+      for (int w = 0; w < 3; ++w)
+        p[w][u] = (uint32_t)__bfloat16_as_ushort(x[w]) | ((uint32_t)__bfloat16_as_ushort(y[w]) << 16);
+    }
+    const long long oi = r.oinner;
+    __nv_bfloat16* dp = dst + q * os0 + d1 * os1 + d2 * os2 + e * oi;
+    if (cnt == 8 && oi == 1 && (((uintptr_t)dp) & 15) == 0) {  // plane strides are multiples of 8 elements
+#pragma unroll
+      for (int w = 0; w < 3; ++w) *(uint4*)(dp + w * plane) = make_uint4(p[w][0], p[w][1], p[w][2], p[w][3]);
+    } else {
+#pragma unroll
+      for (int w = 0; w < 3; ++w)
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (u < cnt) dp[w * plane + u * oi] = __ushort_as_bfloat16((unsigned short)(p[w][u >> 1] >> (16 * (u & 1))));
+    }
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  __shared__ uint32_t wm[8];
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) mx = max(mx, wm[w]);
+    r.amax[chunk - r.chunk_start] = mx;
+  }
+}
+
+// ------------------------------------------------------------------ product
+// The fields of problem p; a single problem's come from the kernel parameters.
+__device__ __forceinline__ F3Fields f3_fields(const F3Args& args, int p) {
+  if (!args.table) return args.one.f;
+  return args.table[p].f;
+}
+
+struct F3Where { int p, b, tm, tn, k; };  // k < 0: out of range, -k is the extent
+
+// meta[p] = (tile_start, tiles_m, tiles_n, k or -k)
+__device__ __forceinline__ F3Where f3_locate(const int4* meta, int num, int t) {
+  int lo = 0, hi = num - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (meta[mid].x <= t) lo = mid; else hi = mid - 1;
+  }
+  const int4 e = meta[lo];
+  F3Where w;
+  w.p = lo;
+  w.k = e.w;
+  const int per = e.y * e.z, lt = t - e.x;
+  w.b = lt / per;
+  band_tile(lt - w.b * per, e.y, e.z, w.tm, w.tn);
+  return w;
+}
+
+// What the epilogue needs of a problem.
+struct F3Out {
+  float* c;          // of the tile's batch
+  const float* bias;
+  long long ldc;
+  int m, n, relu;
+  float alpha, beta;
+  bool plain, c_col;
+};
+
+__device__ __forceinline__ F3Out f3_out(const F3Args& args, int p, int batch) {
+  const F3Fields f = f3_fields(args, p);
+  F3Out o;
+  o.c = f.c + batch * f.c_batch;
+  o.bias = f.bias;
+  o.ldc = f.ldc;
+  o.m = f.m;
+  o.n = f.n;
+  o.relu = f.relu;
+  o.alpha = f.alpha;
+  o.beta = f.beta;
+  o.plain = f.beta == 0.f && !f.bias && !f.relu;
+  o.c_col = f.c_col != 0;
+  return o;
+}
+
+__device__ __forceinline__ float f3_finish(const F3Out& o, float acc, const float* cp, int col) {
+  float v = o.alpha * acc;
+  if (o.plain) return v;
+  if (o.beta != 0.f) v += o.beta * *cp;
+  if (o.bias) v += o.bias[col];
+  if (o.relu) v = v > 0.f ? v : 0.f;
+  return v;
+}
+
+// The FP32 form of one thread's row of the tile: columns [col0, col0 + ncols),
+// one FMA chain over k per output (k_gemm_f32's order).
+__device__ __noinline__ void f3_plain_row(const F3Args& args, int p, int batch, int row, int col0, int ncols) {
+  const F3Fields f = f3_fields(args, p);
+  const F3Out o = f3_out(args, p, batch);
+  if (row >= o.m || col0 >= o.n) return;
+  const __nv_bfloat16* __restrict__ A = f.a + batch * f.a_batch + row * f.a_row;
+  const __nv_bfloat16* __restrict__ B = f.b + batch * f.b_batch;
+  const long long ak = f.a_k, bk = f.b_k, bc = f.b_col, ap = f.a_plane, bpl = f.b_plane;
+  const int end = min(col0 + ncols, o.n);
+  for (int c0 = col0; c0 < end; c0 += 8) {
+    float s[8];
+    const __nv_bfloat16* bp[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      s[u] = 0.f;
+      bp[u] = B + (long long)min(c0 + u, o.n - 1) * bc;
+    }
+    for (int k = 0; k < f.k; ++k) {
+      const float av = f3_join(A + k * ak, ap);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s[u] = fmaf(av, f3_join(bp[u] + k * bk, bpl), s[u]);
+    }
+    for (int u = 0; u < 8 && c0 + u < end; ++u) {
+      const int col = c0 + u;
+      float* cp = o.c + (o.c_col ? row + col * o.ldc : row * o.ldc + col);
+      *cp = f3_finish(o, s[u], cp, col);
+    }
+  }
+}
+
+// One warp's 32 rows x NC columns of C from its accumulators (lane l holds row
+// row0 + l). Row-major C goes through the warp's 32 x 16 buffer, so that each
+// store writes whole 64-byte row segments (4 lanes x 16 bytes, 8 rows); columns
+// of a column-major C are already 32 consecutive elements across the lanes.
+template <int NC>
+__device__ __forceinline__ void f3_store(const F3Out& o, int row0, int col0, int lane, float* stage, const float (&acc)[NC]) {
+  if (row0 >= o.m) return;
+  if (o.c_col) {
+    const bool row_ok = row0 + lane < o.m;
+    float* cp = o.c + row0 + lane + (long long)col0 * o.ldc;
+#pragma unroll
+    for (int j = 0; j < NC; ++j, cp += o.ldc)
+      if (col0 + j < o.n && row_ok) *cp = f3_finish(o, acc[j], cp, col0 + j);
+    return;
+  }
+  const bool vec = ((((uintptr_t)o.c) & 15) == 0) && (o.ldc & 3) == 0 && (o.n & 3) == 0;
+  const int rr = lane >> 2, cc = (lane & 3) * 4;
+  float* const crow = o.c + (long long)(row0 + rr) * o.ldc + col0 + cc;
+#pragma unroll
+  for (int j = 0; j < NC / 16; ++j) {
+    if (col0 + 16 * j >= o.n) break;  // warp-uniform
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *(float4*)(stage + lane * kF3EpiPitch + 4 * q) =
+          make_float4(acc[16 * j + 4 * q], acc[16 * j + 4 * q + 1], acc[16 * j + 4 * q + 2], acc[16 * j + 4 * q + 3]);
+    __syncwarp();
+    float4 x[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) x[s] = *(const float4*)(stage + (8 * s + rr) * kF3EpiPitch + cc);
+    __syncwarp();
+    const int col = col0 + 16 * j + cc;
+    if (vec && o.plain) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+        if (row0 + 8 * s + rr < o.m && col < o.n)
+          *(float4*)(crow + 8 * s * o.ldc + 16 * j) =
+              make_float4(o.alpha * x[s].x, o.alpha * x[s].y, o.alpha * x[s].z, o.alpha * x[s].w);
+    } else {
+#pragma unroll 1
+      for (int e = 0; e < 16; ++e) {
+        const int s = e >> 2, q = e & 3;
+        float v = s == 0 ? (q == 0 ? x[0].x : q == 1 ? x[0].y : q == 2 ? x[0].z : x[0].w)
+                : s == 1 ? (q == 0 ? x[1].x : q == 1 ? x[1].y : q == 2 ? x[1].z : x[1].w)
+                : s == 2 ? (q == 0 ? x[2].x : q == 1 ? x[2].y : q == 2 ? x[2].z : x[2].w)
+                         : (q == 0 ? x[3].x : q == 1 ? x[3].y : q == 2 ? x[3].z : x[3].w);
+        if (row0 + 8 * s + rr < o.m && col + q < o.n) {
+          float* cp = crow + 8 * s * o.ldc + 16 * j + q;
+          *cp = f3_finish(o, v, cp, col + q);
+        }
+      }
+    }
+  }
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void f3_tma(uint8_t* dst, const void* tmap, uint64_t* full, uint32_t full_pair, int x, int y, int z) {
+  if constexpr (PAIR) tma_load_3d_2sm(dst, tmap, full_pair, x, y, z);
+  else tma_load_3d(dst, tmap, full, x, y, z);
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void f3_mma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accum) {
+  if constexpr (PAIR) umma_f16_2sm(d, da, db, idesc, accum);
+  else umma_f16(d, da, db, idesc, accum);
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void f3_commit(uint64_t* bar) {
+  if constexpr (PAIR) umma_commit_2sm(bar, 0x3);
+  else umma_commit(bar);
+}
+
+// Four MMAs (K = 16 each) of one pair of plane tiles; ka, kb: a K step of the
+// descriptors. FIRST: how the first one treats the accumulator: 0 adds to it, 1
+// starts it, 2 scales it by 2^-8.
+template <bool PAIR, int FIRST>
+__device__ __forceinline__ void f3_product(uint32_t d, uint64_t da, uint64_t db, uint32_t ka, uint32_t kb, uint32_t idesc) {
+  if constexpr (FIRST == 2) {
+    if constexpr (PAIR) umma_f16_2sm_shift_d<8>(d, da, db, idesc);
+    else umma_f16_shift_d<8>(d, da, db, idesc);
+  } else {
+    f3_mma<PAIR>(d, da, db, idesc, FIRST == 1 ? 0u : 1u);
+  }
+#pragma unroll
+  for (int kk = 1; kk < 4; ++kk) f3_mma<PAIR>(d, da + kk * ka, db + kk * kb, idesc, 1u);
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void f3_gemm_body(const F3Args& args) {
+  constexpr int BM = PAIR ? 256 : 128, BN = BM;
+  constexpr int NC = BN / 2;  // columns per epilogue warp
+  constexpr int TMEM_COLS = 2 * BN;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  float* epi = (float*)(smem + 2 * kF3Stage);
+  uint64_t* bars = (uint64_t*)(smem + 2 * kF3Stage + kF3EpiWarps * kF3EpiSlot);
+  uint64_t* full = bars;              // [2]
+  uint64_t* empty = bars + 2;         // [2][5]
+  uint64_t* tfull = bars + 12;        // [2]
+  uint64_t* tempty = bars + 14;       // [2]
+  uint32_t* tmem_slot = (uint32_t*)(bars + 16);
+  int4* meta = (int4*)((uint8_t*)bars + 256);
+  volatile uint32_t* status = args.status;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  const bool leader = rank == 0;
+  const int unit = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+  const int units = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int s = 0; s < 2; ++s) {
+        mbar_init(&full[s], 1);
+        for (int e = 0; e < 5; ++e) mbar_init(&empty[5 * s + e], 1);
+        mbar_init(&tfull[s], 1);
+        mbar_init(&tempty[s], (PAIR ? 2 : 1) * kF3EpiWarps);
+      }
+      fence_mbar_init();
+      if (!args.table) {
+        prefetch_tensormap(&args.one.tmap_a);
+        prefetch_tensormap(&args.one.tmap_b);
+      }
+    }
+  } else if (warp == 1) {
+    if constexpr (PAIR) tmem_alloc_2sm(tmem_slot, TMEM_COLS);
+    else tmem_alloc(tmem_slot, TMEM_COLS);
+  } else {
+    // one warp per problem: its tiles, and whether its operands are in range
+    for (int p = warp - 2; p < args.num_problems; p += kF3EpiWarps) {
+      const F3Fields f = f3_fields(args, p);
+      const uint32_t *xa = f.amax_a, *xb = f.amax_b;
+      const int na = f.na, nb = f.nb, k = f.k;
+      uint32_t ma = 0, mb = 0;
+      for (int i = lane; i < max(na, nb); i += 32) {
+        if (i < na) ma = max(ma, xa[i]);
+        if (i < nb) mb = max(mb, xb[i]);
+      }
+      ma = __reduce_max_sync(0xffffffffu, ma);
+      mb = __reduce_max_sync(0xffffffffu, mb);
+      if (lane == 0) meta[p] = make_int4(f.tile_start, f.tiles_m, f.tiles_n, f3_in_range(ma, mb, k) ? k : -k);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if constexpr (PAIR) {
+    __syncwarp();
+    cluster_sync();
+  }
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  // tile of this unit in a round; the same in every lane
+  auto locate = [&](int t0, int round) {
+    F3Where w = f3_locate(meta, args.num_problems, snake_tile_of(t0, round, args.total_tiles, unit, units));
+    w.p = warp_uniform(w.p);
+    w.b = warp_uniform(w.b);
+    w.tm = warp_uniform(w.tm);
+    w.tn = warp_uniform(w.tn);
+    w.k = warp_uniform(w.k);
+    return w;
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ producer
+    uint32_t c = 0;  // chunks so far: stage c & 1
+    bool ok = true;
+    int last_p = -1;
+    for (int t0 = unit, rr = 0; t0 < args.total_tiles && ok; t0 += units, ++rr) {
+      const F3Where w = locate(t0, rr);
+      if (w.k <= 0) continue;
+      const F3Fields f = f3_fields(args, w.p);
+      const CUtensorMap* const map_a = args.table ? &args.table[w.p].tmap_a : &args.one.tmap_a;
+      const CUtensorMap* const map_b = args.table ? &args.table[w.p].tmap_b : &args.one.tmap_b;
+      const bool a_mn = warp_uniform(f.a_mn) != 0, b_mn = warp_uniform(f.b_mn) != 0;
+      const int nb = warp_uniform(f.batch);
+      const int row_a = w.tm * BM + (int)rank * 128, row_b = w.tn * BN + (int)rank * 128;
+      if (args.table && w.p != last_p) {
+        if (elect_one()) {
+          tensormap_acquire(map_a);
+          tensormap_acquire(map_b);
+        }
+        last_p = w.p;
+      }
+      for (int k0 = 0; k0 < w.k && ok; k0 += kF3BK, ++c) {
+        const uint32_t s = c & 1, ph = (c >> 1) & 1;
+        uint8_t* const sa = smem + s * kF3Stage;
+        uint8_t* const sb = sa + 3 * kF3Tile;
+        uint64_t* const fb = &full[s];
+        uint64_t* const eb = &empty[5 * s];
+        const uint32_t fp = PAIR ? mapa_shared(smem_u32(fb), 0) : 0u;
+        auto load_a = [&](int plane) {
+          uint8_t* const dst = sa + plane * kF3Tile;
+          if (a_mn) {
+            f3_tma<PAIR>(dst, map_a, fb, fp, row_a, k0, plane * nb + w.b);
+            f3_tma<PAIR>(dst + kF3BK * 128, map_a, fb, fp, row_a + 64, k0, plane * nb + w.b);
+          } else {
+            f3_tma<PAIR>(dst, map_a, fb, fp, k0, row_a, plane * nb + w.b);
+          }
+        };
+        auto load_b = [&](int plane) {
+          uint8_t* const dst = sb + plane * kF3Tile;
+          if (b_mn) {
+            f3_tma<PAIR>(dst, map_b, fb, fp, row_b, k0, plane * nb + w.b);
+            f3_tma<PAIR>(dst + kF3BK * 128, map_b, fb, fp, row_b + 64, k0, plane * nb + w.b);
+          } else {
+            f3_tma<PAIR>(dst, map_b, fb, fp, k0, row_b, plane * nb + w.b);
+          }
+        };
+        // in the order in which the products hand the tiles back
+        if (!(ok = mbar_wait_warp(&eb[0], ph ^ 1, status, DEV_TIMEOUT_EMPTY))) break;
+        if (elect_one()) {
+          if (leader) mbar_arrive_expect_tx(fb, (PAIR ? 2 : 1) * kF3Stage);
+          load_b(2);
+        }
+        if (!(ok = mbar_wait_warp(&eb[1], ph ^ 1, status, DEV_TIMEOUT_EMPTY))) break;
+        if (elect_one()) load_a(2);
+        if (!(ok = mbar_wait_warp(&eb[2], ph ^ 1, status, DEV_TIMEOUT_EMPTY))) break;
+        if (elect_one()) load_b(1);
+        if (!(ok = mbar_wait_warp(&eb[3], ph ^ 1, status, DEV_TIMEOUT_EMPTY))) break;
+        if (elect_one()) load_a(1);
+        if (!(ok = mbar_wait_warp(&eb[4], ph ^ 1, status, DEV_TIMEOUT_EMPTY))) break;
+        if (elect_one()) {
+          load_a(0);
+          load_b(0);
+        }
+      }
+    }
+    // every issued load has landed and been read before the CTA may exit
+    for (int i = 0; i < 2 && ok; ++i, ++c)
+      for (int e = 0; e < 5 && ok; ++e) ok = mbar_wait_warp(&empty[5 * (c & 1) + e], ((c >> 1) & 1) ^ 1, status, DEV_TIMEOUT_EMPTY);
+    if (lane == 0 && *status != DEV_OK) {
+      const long long t0 = clock64();
+      while (clock64() - t0 < 200000) {}
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer (the pair's leader)
+    if (leader) {
+      uint32_t c = 0;
+      bool ok = true;
+      for (int t0 = unit, rr = 0; t0 < args.total_tiles && ok; t0 += units, ++rr) {
+        const F3Where w = locate(t0, rr);
+        if (w.k <= 0) continue;
+        const F3Fields f = f3_fields(args, w.p);
+        const bool a_mn = warp_uniform(f.a_mn) != 0, b_mn = warp_uniform(f.b_mn) != 0;
+        const uint32_t idesc = make_idesc(BM, BN, 1u, a_mn, b_mn);
+        // descriptors of plane 0's first K step in stage 0; their low words count 16-byte units
+        const uint32_t s0 = smem_u32(smem);
+        const uint64_t da0 = smem_desc_sw128(s0, a_mn ? kF3BK * 128 : 16, 1024);
+        const uint64_t db0 = smem_desc_sw128(s0 + 3 * kF3Tile, b_mn ? kF3BK * 128 : 16, 1024);
+        const uint32_t ka = (a_mn ? 2048 : 32) >> 4, kb = (b_mn ? 2048 : 32) >> 4;
+        constexpr uint32_t P = kF3Tile >> 4;  // to the next plane
+        for (int k0 = 0; k0 < w.k; k0 += kF3BK, ++c) {
+          const uint32_t s = c & 1, ph = (c >> 1) & 1;
+          if (!(ok = mbar_wait_warp(&tempty[s], ph ^ 1, status, DEV_TIMEOUT_TMEM_EMPTY))) break;
+          if (!(ok = mbar_wait_warp(&full[s], ph, status, DEV_TIMEOUT_FULL))) break;
+          tc_fence_after();
+          if (elect_one()) {
+            const uint32_t d = tmem_base + s * BN;
+            const uint64_t da = da0 + s * (kF3Stage >> 4), db = db0 + s * (kF3Stage >> 4);
+            uint64_t* const e = empty + 5 * s;
+            f3_product<PAIR, 1>(d, da, db + 2 * P, ka, kb, idesc);       // a0 b2
+            f3_commit<PAIR>(&e[0]);
+            f3_product<PAIR, 0>(d, da + 2 * P, db, ka, kb, idesc);       // a2 b0
+            f3_commit<PAIR>(&e[1]);
+            f3_product<PAIR, 0>(d, da + P, db + P, ka, kb, idesc);      // a1 b1
+            f3_product<PAIR, 2>(d, da, db + P, ka, kb, idesc);           // a0 b1
+            f3_commit<PAIR>(&e[2]);
+            f3_product<PAIR, 0>(d, da + P, db, ka, kb, idesc);           // a1 b0
+            f3_commit<PAIR>(&e[3]);
+            f3_product<PAIR, 2>(d, da, db, ka, kb, idesc);                // a0 b0
+            f3_commit<PAIR>(&e[4]);
+            f3_commit<PAIR>(&tfull[s]);
+          }
+          __syncwarp();
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ epilogue
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    float* stage = epi + (warp - 2) * (kF3EpiSlot / 4);
+    const uint32_t te[2] = {PAIR ? mapa_shared(smem_u32(&tempty[0]), 0) : 0u, PAIR ? mapa_shared(smem_u32(&tempty[1]), 0) : 0u};
+    uint32_t c = 0;
+    bool ok = true;
+    for (int t0 = unit, rr = 0; t0 < args.total_tiles && ok; t0 += units, ++rr) {
+      const F3Where w = locate(t0, rr);
+      const int row0 = w.tm * BM + (int)rank * 128 + 32 * quarter, col0 = w.tn * BN + half * NC;
+      if (w.k <= 0) {
+        f3_plain_row(args, w.p, w.b, row0 + lane, col0, NC);
+        continue;
+      }
+      const F3Out o = f3_out(args, w.p, w.b);
+      float acc[NC];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) acc[j] = 0.f;
+      for (int k0 = 0; k0 < w.k; k0 += kF3BK, ++c) {
+        const uint32_t s = c & 1, ph = (c >> 1) & 1;
+        const bool got = mbar_wait(&tfull[s], ph, status, DEV_TIMEOUT_TMEM_FULL);
+        if (!(ok = __all_sync(0xffffffffu, got))) break;
+        tc_fence_after();
+        const uint32_t t_row = tmem_base + s * BN + half * NC + ((uint32_t)(32 * quarter) << 16);
+#pragma unroll
+        for (int j = 0; j < NC / 32; ++j) {
+          uint32_t r0[16], r1[16];
+          tmem_ld16_nowait(t_row + 32 * j, r0);
+          tmem_ld16_nowait(t_row + 32 * j + 16, r1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            acc[32 * j + q] = __fadd_rn(acc[32 * j + q], __uint_as_float(r0[q]));
+            acc[32 * j + 16 + q] = __fadd_rn(acc[32 * j + 16 + q], __uint_as_float(r1[q]));
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (PAIR) mbar_arrive_cluster(te[s]);
+          else mbar_arrive(&tempty[s]);
+        }
+      }
+      if (!ok) break;
+      f3_store<NC>(o, row0, col0, lane, stage, acc);
+    }
+  }
+
+  // in a pair the leader's MMAs read the peer's shared memory: neither CTA may
+  // release TMEM or exit before both are done
+  tc_fence_before();
+  __syncthreads();
+  if constexpr (PAIR) {
+    __syncwarp();
+    cluster_sync();
+  }
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    if constexpr (PAIR) tmem_dealloc_2sm(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kF3Threads, 1)
+    f32_gemm_pair_kernel(const __grid_constant__ F3Args args) {
+  f3_gemm_body<true>(args);
+}
+
+__global__ void __launch_bounds__(kF3Threads, 1) f32_gemm_kernel(const __grid_constant__ F3Args args) {
+  f3_gemm_body<false>(args);
+}
+
+}  // namespace bbx

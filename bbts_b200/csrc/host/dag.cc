@@ -7,10 +7,13 @@
 //   STREAM  grouped streaming launches: every add / n-ary reduce / elementwise
 //           node of the wave, and the split first activation as two
 //           element-wise ops (more than 16 reduce inputs chain extra phases)
-//   OTHER   direct calls of the remaining impls (FP32 SIMT matmul, FP32
-//           contraction, FNN ops, softmax, uniform)
+//   OTHER   the remaining FP32 matmuls in one grouped SIMT launch per operand
+//           layout (small ones, and pre-activations: bbx::FmaChain), and direct
+//           calls of the other impls (small FP32 contractions, FNN ops, softmax, uniform)
 //   TC      one grouped tcgen05 launch per operand-layout class: the wave's
-//           block matmuls and contraction matmuls
+//           block matmuls and contraction matmuls; the f32 ones large enough for
+//           the tensor cores (f3_wanted) in one group of their own, which splits
+//           every operand once and then runs all products
 //   POST    one grouped gather launch: contraction outputs whose mode order
 //           needs a final permutation
 // TC groups run on a tensor stream, everything else on a memory stream, and
@@ -38,6 +41,7 @@
 #include <stdexcept>
 #include <string>
 #include "contraction.h"
+#include "f32tc.h"
 #include "runtime.h"
 
 namespace bbx {
@@ -64,6 +68,8 @@ struct node_t {
   ud_impl_t* impl;
   node_kind_t kind;
   bool tc_contract = false;  // bf16 contraction lowered into PRE / TC / POST groups
+  bool f3 = false;           // f32 matmul or contraction of the wave's f32 tensor-core group
+  bool chain = false;        // its f32 products keep the FMA chain
   std::vector<tid_t> ins, outs;
   int asap = 0, height = 0, wave = 0;
   int resource = 1;          // 0 tensor stream, 1 memory stream
@@ -81,6 +87,7 @@ struct tplan_t {
 
 struct opaque_t {
   ud_impl_t* impl;
+  bool chain;
   std::vector<command_param_t> params;
   std::vector<tid_t> ins, outs;
 };
@@ -94,6 +101,8 @@ struct group_t {
   bbx_stream_plan_t* stream_plan = nullptr;
   bbx_tc_plan_t* tc_plan = nullptr;
   bbx::GatherPlan* gather_plan = nullptr;
+  bbx::F3Plan* f3_plan = nullptr;  // G_TC without a tc_plan: the wave's f32 products
+  bbx::F32SimtPlan* simt_plan = nullptr;  // G_OTHER: f32 matmuls of the SIMT kernels
   std::vector<opaque_t> opaque;
   std::vector<int> deps;  // indices of earlier groups this one waits for
   double flops = 0.0;     // algorithmic work of the launch: 2mnk for tensor groups,
@@ -168,6 +177,7 @@ void run_opaque(dag_t* d, opaque_t& o, cudaStream_t st) {
   for (tid_t t : o.ins) ins.push_back(header(d, t));
   for (tid_t t : o.outs) outs.push_back(header(d, t));
   ud_impl_t::tensor_args_t ia(ins), oa(outs);
+  const bbx::FmaChain chain(o.chain);
   o.impl->call_ud(params, ia, oa);
 }
 
@@ -176,8 +186,9 @@ void launch_group(dag_t* d, group_t& g, cudaStream_t st) {
     case G_PRE:
     case G_POST: dag_bbx(bbx::gather_plan_launch(g.gather_plan, st)); break;
     case G_STREAM: dag_bbx(bbx_stream_plan_launch(g.stream_plan, st)); break;
-    case G_TC: dag_bbx(bbx_tc_plan_launch(g.tc_plan, st)); break;
+    case G_TC: dag_bbx(g.f3_plan ? bbx::f3_plan_launch(g.f3_plan, st) : bbx_tc_plan_launch(g.tc_plan, st)); break;
     case G_OTHER:
+      if (g.simt_plan) dag_bbx(bbx::f32_simt_plan_launch(g.simt_plan, st));
       for (auto& o : g.opaque) run_opaque(d, o, st);
       break;
   }
@@ -377,9 +388,20 @@ cparams_t parse_contraction(const command_t& c) {
   return r;
 }
 
+void lower_for_tc(const std::vector<tensor_meta_t>& in_metas, const command_t& c, bbx::ContractionLowering* L) {
+  const cparams_t p = parse_contraction(c);
+  const auto& sl = in_metas[0].as<cu_meta_t>().m();
+  const auto& sr = in_metas[1].as<cu_meta_t>().m();
+  std::vector<long long> dl(sl.dims, sl.dims + sl.rank), dr(sr.dims, sr.dims + sr.rank);
+  dag_bbx(bbx::lower_contraction((int)dl.size(), dl.data(), p.ml.data(), (int)dr.size(), dr.data(), p.mr.data(),
+                                 (int)p.mo.size(), p.mo.data(), true, L));
+}
+
 }  // namespace
 
-dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
+// f32_tc: lower f32 products to the tensor cores, whose operand planes live in the
+// arena; *no_room is set when an arena with them does not fit the device.
+static dag_t* dag_build_as(runtime_t* rt, int policy, int tile_n, bool f32_tc, bool* no_room) {
   auto d = std::make_unique<dag_t>();
   d->rt = rt;
   const tensor_factory_t& tf = *rt->tf;
@@ -396,6 +418,7 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
   }
 
   // ---- nodes, output metas, dependencies
+  const std::unordered_set<command_id_t> keep_chain = pre_activations(rt->commands, *rt->udm);
   std::vector<node_t> nodes;
   std::vector<op_features_t> feats;
   std::unordered_map<tid_t, int> producer;
@@ -414,6 +437,7 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
     n.impl = rt->udm->get_fn_impl(c.fun_id);
     if (!n.impl) throw std::runtime_error("DAG: command " + std::to_string(c.id) + " names an unknown ud impl");
     n.kind = classify(n.impl, c.is_reduce());
+    n.chain = keep_chain.count(c.id) != 0;
     if (c.is_reduce() && n.kind != NK_SUM)
       throw std::runtime_error("DAG: REDUCE is supported for matrix_add over dense / dense_bf16 blocks");
     n.tc_contract = n.kind == NK_CONTRACT && n.impl->impl_name == "b200_contraction_bf16";
@@ -459,9 +483,19 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
       const auto& mb = in_metas[1].as<dense_tensor_meta_t>().m();
       bool ta = params.get_bool_or_default<0>(false), tb = params.get_bool_or_default<1>(false);
       double M = ta ? ma.num_cols : ma.num_rows, K = ta ? ma.num_rows : ma.num_cols, N = tb ? mb.num_rows : mb.num_cols;
+      if (n.kind == NK_SIMT && f32_tc && !n.chain && bbx::f3_wanted((long long)M, (long long)N, (long long)K, 1)) {
+        n.f3 = true;
+        n.resource = 0;
+      }
       n.flops = 2.0 * M * N * K;
       n.bytes = (double)tf.get_payload_size(in_metas[0]) + tf.get_payload_size(in_metas[1]) + tf.get_payload_size(out_metas[0]);
     } else if (n.kind == NK_CONTRACT) {
+      if (!n.tc_contract && f32_tc && !n.chain) {
+        bbx::ContractionLowering L;
+        lower_for_tc(in_metas, c, &L);
+        n.f3 = bbx::f3_contraction_wanted(L);
+        if (n.f3) n.resource = 0;
+      }
       n.flops = 2.0 * (double)hint;
     } else {
       double b = 0;
@@ -522,29 +556,52 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
   struct cstage_t { tid_t lc, rc, ct; bbx::ContractionLowering L; cparams_t p; };
   std::unordered_map<int, cstage_t> cstage;
   tid_t next_stage = -1000000;
+  auto stage = [&](size_t bytes, int wave) {
+    tid_t t = next_stage--;
+    tplan_t tp;
+    std::memset(&tp.meta, 0, sizeof(tp.meta));
+    tp.bytes = bytes;
+    tp.def = tp.last = wave;
+    tp.deleted = true;
+    d->tensors[t] = tp;
+    return t;
+  };
+  auto metas_of = [&](const node_t& n) {
+    std::vector<tensor_meta_t> v;
+    for (tid_t t : n.ins) v.push_back(d->tensors.at(t).meta);
+    return v;
+  };
+  // planes of a wave's f32 operands: a block is split once per wave, whatever products read it
+  std::map<std::pair<int, tid_t>, tid_t> f3_stage;
+  bool any_f3 = false;
   for (int i = 0; i < N; ++i) {
     node_t& n = nodes[i];
-    if (!n.tc_contract) continue;
+    any_f3 = any_f3 || n.f3;
+    if (n.f3 && n.kind == NK_SIMT) {
+      for (tid_t t : n.ins) {
+        const auto key = std::make_pair(n.wave, t);
+        if (f3_stage.count(key)) continue;
+        const auto& m = d->tensors.at(t).meta.as<dense_tensor_meta_t>().m();
+        const tid_t st = stage(bbx::f3_mat_bytes(bbx::f3_dense(nullptr, m.num_rows, m.num_cols, m.num_cols, 1, 0, false)), n.wave);
+        f3_stage[key] = st;
+      }
+      continue;
+    }
+    if (!n.tc_contract && !(n.f3 && n.kind == NK_CONTRACT)) continue;
     cstage_t cs;
     cs.p = parse_contraction(*n.cmd);
-    const auto& sl = d->tensors.at(n.ins[0]).meta.as<cu_meta_t>().m();
-    const auto& sr = d->tensors.at(n.ins[1]).meta.as<cu_meta_t>().m();
-    std::vector<long long> dl(sl.dims, sl.dims + sl.rank), dr(sr.dims, sr.dims + sr.rank);
-    dag_bbx(bbx::lower_contraction((int)dl.size(), dl.data(), cs.p.ml.data(), (int)dr.size(), dr.data(),
-                                   cs.p.mr.data(), (int)cs.p.mo.size(), cs.p.mo.data(), true, &cs.L));
-    auto stage = [&](size_t bytes) {
-      tid_t t = next_stage--;
-      tplan_t tp;
-      std::memset(&tp.meta, 0, sizeof(tp.meta));
-      tp.bytes = bytes;
-      tp.def = tp.last = n.wave;
-      tp.deleted = true;
-      d->tensors[t] = tp;
-      return t;
-    };
-    cs.lc = stage((size_t)(cs.L.lc_elems * 2 + 16));
-    cs.rc = stage((size_t)(cs.L.rc_elems * 2 + 16));
-    cs.ct = cs.L.direct ? TID_NONE : stage((size_t)(cs.L.nb * cs.L.nn * cs.L.nm * 4));
+    lower_for_tc(metas_of(n), *n.cmd, &cs.L);
+    size_t lbytes = (size_t)(cs.L.lc_elems * 2 + 16), rbytes = (size_t)(cs.L.rc_elems * 2 + 16);
+    if (n.f3) {
+      bbx::F3Mat ml, mr;
+      bbx::F3Spec sp;
+      bbx::f3_contraction(cs.L, nullptr, nullptr, nullptr, cs.p.alpha, &ml, &mr, &sp);
+      lbytes = bbx::f3_mat_bytes(ml);
+      rbytes = bbx::f3_mat_bytes(mr);
+    }
+    cs.lc = stage(lbytes, n.wave);
+    cs.rc = stage(rbytes, n.wave);
+    cs.ct = cs.L.direct ? TID_NONE : stage((size_t)(cs.L.nb * cs.L.nn * cs.L.nm * 4), n.wave);
     cstage[i] = cs;
   }
 
@@ -589,7 +646,20 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
     offsets[tid] = off;
     arena = std::max(arena, off + bytes);
   }
-  if (arena) dag_cuda(cudaMalloc(&d->arena, arena), "cudaMalloc(DAG arena)");
+  if (arena) {
+    cudaError_t e = cudaMalloc(&d->arena, arena);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      bbx::scratch_trim();
+      e = cudaMalloc(&d->arena, arena);
+    }
+    if (e == cudaErrorMemoryAllocation && no_room && any_f3) {
+      cudaGetLastError();
+      *no_room = true;
+      return nullptr;
+    }
+    dag_cuda(e, "cudaMalloc(DAG arena)");
+  }
   d->arena_bytes = arena;
   for (auto& kv : offsets) d->tensors[kv.first].payload = (char*)d->arena + kv.second;
   for (auto& kv : d->tensors) {
@@ -610,7 +680,7 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
   // bulk-staged gather (its shared memory) would keep off those SMs
   std::vector<char> wave_mm(nw, 0);
   for (int i = 0; i < N; ++i)
-    if (nodes[i].kind == NK_TC) wave_mm[nodes[i].wave] = 1;
+    if (nodes[i].kind == NK_TC || nodes[i].f3) wave_mm[nodes[i].wave] = 1;
   for (int w = 0; w < nw; ++w) {
     auto& ids = by_wave[w];
     const bool bulk_gather = !wave_mm[w] && !(w > 0 && wave_mm[w - 1]);
@@ -623,13 +693,94 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
     std::vector<std::vector<bbx_stream_op_t>> phases(1);
     std::vector<std::pair<std::vector<tid_t>, std::vector<tid_t>>> phase_rw(1);
     std::vector<bbx::GatherRec> pre, post;
-    group_t gpre{G_PRE, w}, gpost{G_POST, w}, gother{G_OTHER, w};
+    group_t gpre{G_PRE, w}, gpost{G_POST, w}, gother{G_OTHER, w}, gf3{G_TC, w};
+    group_t gsimt{G_OTHER, w};
+    std::vector<bbx::F32SimtSpec> simt;
+    std::vector<bbx::F3Mat> f3_mats;
+    std::vector<bbx::F3Spec> f3_specs;
+    std::map<std::pair<tid_t, bool>, int> f3_of;  // (operand block, read MN-major) -> f3_mats
+    auto f3_add = [&](bbx::F3Mat m, tid_t planes) {
+      m.ws = d->tensors.at(planes).payload;
+      gf3.writes.push_back(planes);
+      f3_mats.push_back(m);
+      return (int)f3_mats.size() - 1;
+    };
     for (int i : ids) {
       node_t& n = nodes[i];
       const command_t& c = *n.cmd;
       ud_impl_t::tensor_params_t params;
       params._params = c.get_parameters();
-      if (n.kind == NK_TC) {
+      if (n.f3 && n.kind == NK_SIMT) {
+        const bool tr[2] = {params.get_bool_or_default<0>(false) != 0, params.get_bool_or_default<1>(false) != 0};
+        bbx::F3Spec q;
+        const auto& mc = d->tensors.at(n.outs[0]).meta.as<dense_tensor_meta_t>().m();
+        int id[2];
+        for (int j = 0; j < 2; ++j) {
+          const auto& t = d->tensors.at(n.ins[j]);
+          const auto& m = t.meta.as<dense_tensor_meta_t>().m();
+          // MN-major where the rows run along K: a transposed A, a plain B. One block's
+          // planes serve both uses; the use only picks how the product reads them.
+          const bool mn = j == 0 ? tr[0] : !tr[1];
+          const auto it = f3_of.find({n.ins[j], mn});
+          if (it != f3_of.end()) {
+            id[j] = it->second;
+          } else {
+            bbx::F3Mat x = bbx::f3_dense((const float*)t.payload, m.num_rows, m.num_cols, m.num_cols, 1, 0, mn);
+            x.split = f3_of.find({n.ins[j], !mn}) == f3_of.end();
+            id[j] = f3_add(x, f3_stage.at({w, n.ins[j]}));
+            f3_of[{n.ins[j], mn}] = id[j];
+          }
+          if (j == 0) q.k = (int)(tr[0] ? m.num_rows : m.num_cols);
+        }
+        q.a = id[0]; q.b = id[1];
+        q.m = (int)mc.num_rows; q.n = (int)mc.num_cols;
+        q.c = (float*)d->tensors.at(n.outs[0]).payload;
+        q.ldc = mc.num_cols;
+        f3_specs.push_back(q);
+        gf3.flops += n.flops;
+        gf3.bytes += n.bytes;
+        gf3.reads.insert(gf3.reads.end(), n.ins.begin(), n.ins.end());
+        gf3.writes.push_back(n.outs[0]);
+      } else if (n.kind == NK_SIMT) {
+        const auto &ta_ = d->tensors.at(n.ins[0]), &tb_ = d->tensors.at(n.ins[1]), &tc_ = d->tensors.at(n.outs[0]);
+        const auto &ma = ta_.meta.as<dense_tensor_meta_t>().m(), &mb = tb_.meta.as<dense_tensor_meta_t>().m();
+        const auto& mc = tc_.meta.as<dense_tensor_meta_t>().m();
+        bbx::F32SimtSpec q{};
+        q.a = (const float*)ta_.payload; q.b = (const float*)tb_.payload; q.c = (float*)tc_.payload;
+        q.trans_a = params.get_bool_or_default<0>(false) != 0;
+        q.trans_b = params.get_bool_or_default<1>(false) != 0;
+        q.m = (int)mc.num_rows; q.n = (int)mc.num_cols;
+        q.k = (int)(q.trans_a ? ma.num_rows : ma.num_cols);
+        q.lda = ma.num_cols; q.ldb = mb.num_cols; q.ldc = mc.num_cols;
+        simt.push_back(q);
+        gsimt.flops += n.flops;
+        gsimt.reads.insert(gsimt.reads.end(), n.ins.begin(), n.ins.end());
+        gsimt.writes.push_back(n.outs[0]);
+      } else if (n.f3) {
+        cstage_t& cs = cstage.at(i);
+        auto& L = cs.L;
+        bbx::F3Mat ml, mr;
+        bbx::F3Spec q;
+        float* C = (float*)d->tensors.at(L.direct ? n.outs[0] : cs.ct).payload;
+        bbx::f3_contraction(L, (const float*)d->tensors.at(n.ins[0]).payload, (const float*)d->tensors.at(n.ins[1]).payload, C,
+                            cs.p.alpha, &ml, &mr, &q);
+        const int id[2] = {f3_add(ml, cs.lc), f3_add(mr, cs.rc)};
+        q.a = id[q.a];
+        q.b = id[q.b];
+        f3_specs.push_back(q);
+        gf3.flops += n.flops;
+        gf3.bytes += 4.0 * ((double)L.nl + (double)L.nr + (double)L.no);
+        gf3.reads.insert(gf3.reads.end(), n.ins.begin(), n.ins.end());
+        gf3.writes.push_back(L.direct ? n.outs[0] : cs.ct);
+        if (!L.direct) {
+          bbx::GatherRec ro{};
+          ro.a = L.go; ro.src = C; ro.dst = d->tensors.at(n.outs[0]).payload;
+          ro.dst_bf16 = 0; ro.n = L.no;
+          post.push_back(ro);
+          gpost.reads.push_back(cs.ct);
+          gpost.writes.push_back(n.outs[0]);
+        }
+      } else if (n.kind == NK_TC) {
         auto& ta_ = d->tensors.at(n.ins[0]);
         auto& tb_ = d->tensors.at(n.ins[1]);
         auto& tc_ = d->tensors.at(n.outs[0]);
@@ -758,6 +909,7 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
       } else {
         opaque_t o;
         o.impl = n.impl;
+        o.chain = n.chain;
         auto pl = c.get_parameters();
         o.params.assign(pl.begin(), pl.end());
         o.ins = n.ins;
@@ -814,6 +966,11 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
       d->groups.push_back(std::move(g));
       d->stats.stream_launches++;
     }
+    if (!simt.empty()) {
+      dag_bbx(bbx::f32_simt_plan_create(simt.data(), (int)simt.size(), &gsimt.simt_plan));
+      d->groups.push_back(std::move(gsimt));
+      d->stats.opaque_launches++;
+    }
     if (!gother.opaque.empty()) {
       d->stats.opaque_launches += (int)gother.opaque.size();
       d->groups.push_back(std::move(gother));
@@ -829,6 +986,11 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
       g.reads = tc_rw[kv.first].first;
       g.writes = tc_rw[kv.first].second;
       d->groups.push_back(std::move(g));
+      d->stats.tc_launches++;
+    }
+    if (!f3_specs.empty()) {
+      dag_bbx(bbx::f3_plan_create(f3_mats.data(), (int)f3_mats.size(), f3_specs.data(), (int)f3_specs.size(), &gf3.f3_plan));
+      d->groups.push_back(std::move(gf3));
       d->stats.tc_launches++;
     }
     if (!post.empty()) {
@@ -924,6 +1086,12 @@ dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
   return d.release();
 }
 
+dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
+  bool no_room = false;
+  dag_t* d = dag_build_as(rt, policy, tile_n, true, &no_room);
+  return no_room ? dag_build_as(rt, policy, tile_n, false, nullptr) : d;
+}
+
 void dag_launch(dag_t* d, cudaStream_t st) { dag_cuda(cudaGraphLaunch(d->exec, st), "cudaGraphLaunch"); }
 
 // Replays every group on its own, one after another on `st`, bracketed by
@@ -962,6 +1130,8 @@ void dag_destroy(dag_t* d) {
     if (g.stream_plan) bbx_stream_plan_destroy(g.stream_plan);
     if (g.tc_plan) bbx_tc_plan_destroy(g.tc_plan);
     if (g.gather_plan) bbx::gather_plan_destroy(g.gather_plan);
+    if (g.f3_plan) bbx::f3_plan_destroy(g.f3_plan);
+    if (g.simt_plan) bbx::f32_simt_plan_destroy(g.simt_plan);
   }
   if (d->arena) cudaFree(d->arena);
   for (void* p : d->persistent) cudaFree(p);

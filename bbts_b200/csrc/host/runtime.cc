@@ -1,5 +1,6 @@
 // Runtime: block storage, per-op runner and the grouped DAG executor.
 #include "runtime.h"
+#include "f32tc.h"
 
 #include <fcntl.h>
 #include <unistd.h>
@@ -245,10 +246,23 @@ void block_storage_t::_make_room(size_t need, cudaStream_t st) {
   }
 }
 
+// A block from the storage's pool; when the device is out of memory, once more
+// after the library's scratch pool has given back what it keeps.
+static void* pool_block(size_t bytes, cudaMemPool_t pool, cudaStream_t st, const char* what) {
+  void* p = nullptr;
+  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, st);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    bbx::scratch_trim();
+    e = cudaMallocFromPoolAsync(&p, bytes, pool, st);
+  }
+  cuda_ok(e, what);
+  return p;
+}
+
 void block_storage_t::_reload(block_t& b, cudaStream_t st) {
   _make_room(b.bytes, st);
-  void* p = nullptr;
-  cuda_ok(cudaMallocFromPoolAsync(&p, b.bytes, _pool, st), "cudaMallocFromPoolAsync(reload)");
+  void* p = pool_block(b.bytes, _pool, st, "cudaMallocFromPoolAsync(reload)");
   b.payload = p;
   if (b.host_valid) {
     wait_on(st, b.copied);
@@ -279,8 +293,7 @@ tensor_t* block_storage_t::create(tid_t tid, const tensor_meta_t& meta, cudaStre
   }
   size_t bytes = _tf->get_payload_size(meta);
   _make_room(bytes, st);
-  void* p = nullptr;
-  if (bytes) cuda_ok(cudaMallocFromPoolAsync(&p, bytes, _pool, st), "cudaMallocFromPoolAsync(block)");
+  void* p = bytes ? pool_block(bytes, _pool, st, "cudaMallocFromPoolAsync(block)") : nullptr;
   auto& b = _blocks[tid];
   b.header.reset(new char[sizeof(tensor_meta_t)]);
   std::memcpy(b.header.get(), &meta, sizeof(tensor_meta_t));
@@ -596,8 +609,29 @@ op_features_t features_of(const tensor_factory_t& tfac, const command_t& cmd, ud
   return f;
 }
 
+std::unordered_set<command_id_t> pre_activations(const std::vector<command_ptr_t>& commands, udf_manager_t& udm) {
+  std::unordered_set<command_id_t> found;
+  std::unordered_set<tid_t> reach;
+  for (size_t i = commands.size(); i-- > 0;) {
+    const command_t& c = *commands[i];
+    if (c.is_delete()) continue;
+    const ud_impl_t* impl = udm.get_fn_impl(c.fun_id);
+    if (!impl) continue;
+    const std::string& u = impl->ud_name;
+    bool out = false;
+    for (size_t j = 0; j < c.get_num_outputs(); ++j) out = out || reach.count(c.get_output(j).tid);
+    if (out) found.insert(c.id);
+    const bool relu = u.find("relu") != std::string::npos;
+    const bool add = u == "matrix_add" || u == "ffnn_add" || u == "matrix_weighted_sum" || u == "ffnn_weighted_sum";
+    if (relu || (add && out))
+      for (size_t j = 0; j < c.get_num_inputs(); ++j) reach.insert(c.get_input(j).tid);
+  }
+  return found;
+}
+
 // Executes one APPLY / REDUCE on the runtime stream (the per-op path).
-void execute_command(runtime_t& rt, command_t& cmd, cudaStream_t st) {
+void execute_command(runtime_t& rt, command_t& cmd, cudaStream_t st, bool keep_chain) {
+  const bbx::FmaChain chain(keep_chain);
   ud_impl_t* impl = rt.udm->get_fn_impl(cmd.fun_id);
   if (!impl) throw std::runtime_error("command " + std::to_string(cmd.id) + ": unknown ud impl");
   ud_impl_t::tensor_params_t params;
@@ -751,6 +785,7 @@ void runtime_t::run_per_op(int policy, std::vector<std::pair<op_features_t, floa
     if (!rs.queue_command(c->clone())) throw std::runtime_error("reservation station rejected command " + std::to_string(c->id));
   }
   rs.execute_scheduled_async();
+  const std::unordered_set<command_id_t> keep_chain = pre_activations(commands, *udm);
 
   // ---- worker streams (one = the runtime stream itself)
   const int K = record ? 1 : std::max(1, std::min(workers, 16));
@@ -859,7 +894,7 @@ void runtime_t::run_per_op(int policy, std::vector<std::pair<op_features_t, floa
     }
     storage->begin_command();
     try {
-      execute_command(*this, *cmd, s);
+      execute_command(*this, *cmd, s, keep_chain.count(cmd->id) != 0);
     } catch (...) {
       storage->end_command(s);
       throw;

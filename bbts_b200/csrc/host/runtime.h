@@ -11,6 +11,7 @@
 #include <mutex>
 #include <string>
 #include <unordered_map>
+#include <unordered_set>
 #include <vector>
 #include "bbts_b200.h"
 #include "command.h"
@@ -208,7 +209,10 @@ node_kind_t classify(const ud_impl_t* impl, bool is_reduce);
 op_features_t features_of(const tensor_factory_t& tf, const command_t& cmd, ud_impl_t* impl,
                           std::vector<tensor_meta_t> in_metas, size_t* hint_out);
 int elem_of(const tensor_factory_t& tf, tfid_t id);
-void execute_command(runtime_t& rt, command_t& cmd, cudaStream_t st);
+// Ids of the commands whose result reaches a ReLU, directly or through adds.
+std::unordered_set<command_id_t> pre_activations(const std::vector<command_ptr_t>& commands, udf_manager_t& udm);
+// keep_chain: the command's f32 products keep the FMA chain (bbx::FmaChain).
+void execute_command(runtime_t& rt, command_t& cmd, cudaStream_t st, bool keep_chain);
 
 dag_t* dag_build(runtime_t* rt, int policy, int tile_n);
 // Recording of the autotuner's timings as learned-tile training samples
