@@ -236,8 +236,25 @@ int launch(const F3Args& args, Shape shape, int sms, cudaStream_t st) {
   return e == cudaSuccess ? BBX_OK : set_error(BBX_ERR_CUDA, "f32_gemm: %s", cudaGetErrorString(e));
 }
 
-int launch_split(const F3SplitArgs& args, int chunks, cudaStream_t st) {
-  k_f32_split<<<chunks, 256, 0, st>>>(args);
+// The split kernel of a record.
+enum SplitKind { GENERAL = 0, ROWS = 1, FLAT = 2 };
+bool rows_ok(const F3Split& r) {
+  if (r.rank_s != 0 || r.inner != 1 || r.oinner != 1 || r.plane % 8 != 0 || r.items >= (1ll << 30)) return false;
+  // a row's last piece is written whole: the row stride has to leave it room
+  const bool one_row = r.items == (r.len + 7) / 8;
+  return r.odims[0] == 1 && r.odims[1] == 1 && r.ostride[2] % 8 == 0 && r.istride[2] >= 0 && r.len < (1ll << 31) &&
+         (one_row ? r.plane : r.ostride[2]) >= (r.len + 7) / 8 * 8;
+}
+SplitKind split_kind(const F3Split& r) {
+  if (!rows_ok(r)) return GENERAL;
+  return r.items == r.len / 8 && r.len % 8 == 0 && (((uintptr_t)r.src) & 15) == 0 ? FLAT : ROWS;
+}
+
+int launch_split(const F3SplitArgs& args, int chunks, int kind, cudaStream_t st) {
+  if (chunks == 0) return BBX_OK;
+  if (kind == FLAT) k_f32_split_flat<<<chunks, 256, 0, st>>>(args);
+  else if (kind == ROWS) k_f32_split_rows<<<chunks, 256, 0, st>>>(args);
+  else k_f32_split<<<chunks, 256, 0, st>>>(args);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? BBX_OK : set_error(BBX_ERR_CUDA, "k_f32_split: %s", cudaGetErrorString(e));
 }
@@ -274,20 +291,22 @@ int f3_run(const F3Mat* mats, const F3Spec& spec, void* stream) {
   F3SplitArgs sp;
   std::memset(&sp, 0, sizeof(sp));
   int chunks = 0;
+  int kind = FLAT;  // one launch: the most general kernel of the two (a flat record is also one of rows)
   for (int i : {spec.a, spec.b}) {
-    sp.inl[sp.count++] = split_record(mats[i], chunks);
+    sp.inl[sp.count] = split_record(mats[i], chunks);
+    kind = std::min(kind, (int)split_kind(sp.inl[sp.count++]));
     chunks += (int)chunks_of(mats[i]).count;
     if (spec.a == spec.b) break;
   }
-  rc = launch_split(sp, chunks, (cudaStream_t)stream);
+  rc = launch_split(sp, chunks, kind, (cudaStream_t)stream);
   return rc ? rc : launch(args, shape, sms, (cudaStream_t)stream);
 }
 
 struct F3Plan {
   struct Part { int first, count, tiles, shape; };
   F3Problem* d_problems = nullptr;
-  F3Split* d_splits = nullptr;
-  int n_splits = 0, chunks = 0;
+  F3Split* d_splits = nullptr;     // flat records, row records, the others
+  int n_splits[3] = {0, 0, 0}, chunks[3] = {0, 0, 0};  // by SplitKind
   std::vector<Part> parts;
 };
 
@@ -299,12 +318,15 @@ int f3_plan_create(const F3Mat* mats, int n_mats, const F3Spec* specs, int n_spe
   if (rc) return rc;
   std::unique_ptr<F3Plan, void (*)(F3Plan*)> p(new F3Plan(), f3_plan_destroy);
   std::vector<F3Split> splits;
-  for (int i = 0; i < n_mats; ++i) {
-    if (!mats[i].split) continue;
-    splits.push_back(split_record(mats[i], p->chunks));
-    p->chunks += (int)chunks_of(mats[i]).count;
-  }
-  p->n_splits = (int)splits.size();
+  for (int kind : {FLAT, ROWS, GENERAL})
+    for (int i = 0; i < n_mats; ++i) {
+      if (!mats[i].split) continue;
+      const F3Split r = split_record(mats[i], p->chunks[kind]);
+      if (split_kind(r) != kind) continue;
+      splits.push_back(r);
+      p->chunks[kind] += (int)chunks_of(mats[i]).count;
+      p->n_splits[kind]++;
+    }
   // descending K: the longest tiles first, the shortest even out the end
   std::vector<int> order(n_specs);
   for (int i = 0; i < n_specs; ++i) order[i] = i;
@@ -338,11 +360,16 @@ int f3_plan_launch(F3Plan* p, void* stream) {
   int sms = 148;
   int rc = device_status_and_sms(&status, &sms);
   if (rc) return rc;
-  F3SplitArgs sp;
-  std::memset(&sp, 0, sizeof(sp));
-  sp.table = p->d_splits;
-  sp.count = p->n_splits;
-  rc = launch_split(sp, p->chunks, (cudaStream_t)stream);
+  int first = 0;
+  for (int kind : {FLAT, ROWS, GENERAL}) {
+    F3SplitArgs sp;
+    std::memset(&sp, 0, sizeof(sp));
+    sp.table = p->d_splits + first;
+    sp.count = p->n_splits[kind];
+    first += sp.count;
+    rc = launch_split(sp, p->chunks[kind], kind, (cudaStream_t)stream);
+    if (rc) return rc;
+  }
   for (const auto& part : p->parts) {
     if (rc) return rc;
     F3Args args;

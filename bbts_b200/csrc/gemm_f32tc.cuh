@@ -159,20 +159,137 @@ __device__ __forceinline__ float f3_join(const __nv_bfloat16* p, long long plane
   return __fadd_rn(__bfloat162float(p[0]), lo);
 }
 
-// Chunk blockIdx.x of the launch: its record's items [i0, i1), eight elements
-// of one row each. 4 bytes read and 6 written per element: HBM-bound; 16-byte
-// loads where the row starts on a 16-byte boundary, 16-byte stores of the planes
-// where the row of the planes does. Each CTA writes the maximum of |x| over its
-// chunk as one word, so no counter has to be cleared before the launch.
-__global__ void __launch_bounds__(256) k_f32_split(const __grid_constant__ F3SplitArgs args) {
-  const int chunk = blockIdx.x;
-  int lo = 0, hi = args.count - 1;
+// The planes of eight elements as 16-byte pieces, and the maximum of their magnitudes.
+__device__ __forceinline__ void f3_split8(const float (&v)[8], uint4 (&p)[3], uint32_t& mx) {
+  uint32_t w[3][4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    __nv_bfloat16 x[3], y[3];
+    mx = max(mx, max(__float_as_uint(v[2 * u]) & 0x7FFFFFFFu, __float_as_uint(v[2 * u + 1]) & 0x7FFFFFFFu));
+    f3_split1(v[2 * u], x[0], x[1], x[2]);
+    f3_split1(v[2 * u + 1], y[0], y[1], y[2]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      w[q][u] = (uint32_t)__bfloat16_as_ushort(x[q]) | ((uint32_t)__bfloat16_as_ushort(y[q]) << 16);
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q) p[q] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+}
+
+// Each CTA writes the maximum of |x| over its chunk as one word, so no counter
+// has to be cleared before the launch. All 256 threads.
+__device__ __forceinline__ void f3_chunk_max(uint32_t mx, uint32_t* out) {
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  __shared__ uint32_t wm[8];
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) mx = max(mx, wm[w]);
+    *out = mx;
+  }
+}
+
+__device__ __forceinline__ const F3Split& f3_split_record(const F3SplitArgs& args, int chunk) {
   const F3Split* const recs = args.table ? args.table : args.inl;
+  int lo = 0, hi = args.count - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (recs[mid].chunk_start <= chunk) lo = mid; else hi = mid - 1;
   }
-  const F3Split& r = recs[lo];
+  return recs[lo];
+}
+
+// Chunk blockIdx.x of the launch: its record's items [i0, i1), eight elements
+// each. 4 bytes read and 6 written per element: HBM-bound.
+// Flat records (a whole number of items, contiguous and 16-byte aligned on both
+// sides: every block whose row length is a multiple of 8): two items a thread
+// in flight, 16-byte accesses, few registers so that 48 warps fit an SM. The general form
+// below moved the same records at 2.5 TB/s (64-bit index arithmetic, 80 registers).
+__global__ void __launch_bounds__(256, 6) k_f32_split_flat(const __grid_constant__ F3SplitArgs args) {
+  const F3Split& r = f3_split_record(args, blockIdx.x);
+  const float* __restrict__ src = r.src;
+  __nv_bfloat16* const dst = r.dst;
+  const long long plane = r.plane, per = r.items_per_chunk;
+  uint32_t* const out = r.amax + (blockIdx.x - r.chunk_start);
+  const long long i0 = (blockIdx.x - r.chunk_start) * per;
+  const int n = (int)min(per, r.items - i0);
+  const float4* const sp = (const float4*)src + 2 * i0;
+  uint4* const dp = (uint4*)dst + i0;
+  const long long pw = plane / 8;
+  uint32_t mx = 0;
+  for (int it = threadIdx.x; it < n; it += 512) {
+    const bool two = it + 256 < n;
+    const float4 a = __ldg(sp + 2 * it), b = __ldg(sp + 2 * it + 1);
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f), d = c;
+    if (two) {
+      c = __ldg(sp + 2 * it + 512);
+      d = __ldg(sp + 2 * it + 513);
+    }
+    uint4 p[3];
+    f3_split8({a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, p, mx);
+#pragma unroll
+    for (int w = 0; w < 3; ++w) dp[it + w * pw] = p[w];
+    if (two) {
+      f3_split8({c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w}, p, mx);
+#pragma unroll
+      for (int w = 0; w < 3; ++w) dp[it + 256 + w * pw] = p[w];
+    }
+  }
+  f3_chunk_max(mx, out);
+}
+
+// Row records: rows of consecutive elements on both sides, one row stride each,
+// 16-byte aligned rows in the planes (pitches are multiples of 8), any alignment in the source.
+// An item's eight elements come from the two or three aligned 16-byte pieces that
+// hold them (a lane's eight element loads touched each sector eight times: rows of a
+// contraction's operands moved at 1.7 TB/s), except at the ends of the tensor,
+// where a piece could reach outside it.
+__global__ void __launch_bounds__(256, 5) k_f32_split_rows(const __grid_constant__ F3SplitArgs args) {
+  const F3Split& r = f3_split_record(args, blockIdx.x);
+  const float* __restrict__ src = r.src;
+  __nv_bfloat16* const dst = r.dst;
+  const long long plane = r.plane, istr = r.istride[2], ostr = r.ostride[2];
+  uint32_t* const out = r.amax + (blockIdx.x - r.chunk_start);
+  const uint32_t len = (uint32_t)r.len, per_row = (len + 7) / 8;
+  const uint32_t i0 = (uint32_t)((blockIdx.x - r.chunk_start) * r.items_per_chunk);
+  const uint32_t i1 = (uint32_t)min((long long)i0 + r.items_per_chunk, r.items);
+  const float* const last = src + (r.odims[2] - 1) * istr + len;  // one past the tensor
+  uint32_t mx = 0;
+  for (uint32_t it = i0 + threadIdx.x; it < i1; it += 256) {
+    const uint32_t row = it / per_row, e = (it - row * per_row) * 8;
+    const int cnt = (int)min(8u, len - e);
+    const float* const sp = src + row * istr + e;
+    const int mis = (int)(((uintptr_t)sp >> 2) & 3);
+    float v[8];
+    if (sp - mis >= src && sp - mis + 12 <= last) {
+      const float4* const w = (const float4*)(sp - mis);
+      const float4 a = __ldg(w), b = __ldg(w + 1), c = mis ? __ldg(w + 2) : make_float4(0.f, 0.f, 0.f, 0.f);
+      float x[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+#pragma unroll
+      for (int u = 0; u < 11; ++u) x[u] = (mis & 1) ? x[u + 1] : x[u];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = (mis & 2) ? x[u + 2] : x[u];
+#pragma unroll
+      for (int u = 1; u < 8; ++u) v[u] = u < cnt ? v[u] : 0.f;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = u < cnt ? __ldg(sp + u) : 0.f;
+    }
+    uint4 p[3];
+    f3_split8(v, p, mx);
+    __nv_bfloat16* const dp = dst + row * ostr + e;
+    // a row's last piece ends in its padding (pitch >= len rounded up to 8): zeros there
+#pragma unroll
+    for (int w = 0; w < 3; ++w) *(uint4*)(dp + w * plane) = p[w];
+  }
+  f3_chunk_max(mx, out);
+}
+
+// Any record: strided rows, gathers, summed modes, unaligned rows.
+__global__ void __launch_bounds__(256) k_f32_split(const __grid_constant__ F3SplitArgs args) {
+  const int chunk = blockIdx.x;
+  const F3Split& r = f3_split_record(args, chunk);
   const float* __restrict__ src = r.src;
   __nv_bfloat16* const dst = r.dst;
   const long long plane = r.plane, len = r.len, inner = r.inner;
@@ -235,39 +352,24 @@ __global__ void __launch_bounds__(256) k_f32_split(const __grid_constant__ F3Spl
 #pragma unroll
       for (int u = 0; u < 8; ++u) v[u] = u < cnt ? __ldg(sp + u * inner) : 0.f;
     }
-    uint32_t p[3][4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      __nv_bfloat16 x[3], y[3];
-      mx = max(mx, max(__float_as_uint(v[2 * u]) & 0x7FFFFFFFu, __float_as_uint(v[2 * u + 1]) & 0x7FFFFFFFu));
-      f3_split1(v[2 * u], x[0], x[1], x[2]);
-      f3_split1(v[2 * u + 1], y[0], y[1], y[2]);
-#pragma unroll
-      for (int w = 0; w < 3; ++w)
-        p[w][u] = (uint32_t)__bfloat16_as_ushort(x[w]) | ((uint32_t)__bfloat16_as_ushort(y[w]) << 16);
-    }
+    uint4 p[3];
+    f3_split8(v, p, mx);
     const long long oi = r.oinner;
     __nv_bfloat16* dp = dst + q * os0 + d1 * os1 + d2 * os2 + e * oi;
     if (cnt == 8 && oi == 1 && (((uintptr_t)dp) & 15) == 0) {  // plane strides are multiples of 8 elements
 #pragma unroll
-      for (int w = 0; w < 3; ++w) *(uint4*)(dp + w * plane) = make_uint4(p[w][0], p[w][1], p[w][2], p[w][3]);
+      for (int w = 0; w < 3; ++w) *(uint4*)(dp + w * plane) = p[w];
     } else {
 #pragma unroll
-      for (int w = 0; w < 3; ++w)
+      for (int w = 0; w < 3; ++w) {
+        const uint32_t x[4] = {p[w].x, p[w].y, p[w].z, p[w].w};
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-          if (u < cnt) dp[w * plane + u * oi] = __ushort_as_bfloat16((unsigned short)(p[w][u >> 1] >> (16 * (u & 1))));
+          if (u < cnt) dp[w * plane + u * oi] = __ushort_as_bfloat16((unsigned short)(x[u >> 1] >> (16 * (u & 1))));
+      }
     }
   }
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  __shared__ uint32_t wm[8];
-  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int w = 1; w < 8; ++w) mx = max(mx, wm[w]);
-    r.amax[chunk - r.chunk_start] = mx;
-  }
+  f3_chunk_max(mx, r.amax + (chunk - r.chunk_start));
 }
 
 // ------------------------------------------------------------------ product
