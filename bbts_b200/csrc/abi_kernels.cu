@@ -228,9 +228,9 @@ static int get_encode_fn(EncodeTiledFn* fn) {
 }
 
 // 2-D map over a row-major matrix with `rows` rows of `cols` elements and pitch
-// `ld` elements; box = box_cols x box_rows, 128-byte swizzle, zero OOB fill.
+// `ld` elements; box = box_cols x box_rows, zero OOB fill.
 static int make_map(CUtensorMap* map, const void* base, int dtype, long long rows, long long cols,
-                    long long ld, int box_cols, int box_rows, bool swizzle = true) {
+                    long long ld, int box_cols, int box_rows, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn enc = nullptr;
   int rc = get_encode_fn(&enc);
   if (rc) return rc;
@@ -243,7 +243,7 @@ static int make_map(CUtensorMap* map, const void* base, int dtype, long long row
   cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return set_error(BBX_ERR_INVALID,
@@ -372,7 +372,8 @@ static int build_problem(int in_dtype, const bbx_tc_problem_t& q, int bn_code, T
     if (out->flags & EPI_BETA) return set_error(BBX_ERR_UNSUPPORTED, "column-major C with beta");
     out->flags |= EPI_C_TRANS;
     if ((((uintptr_t)q.c) & 15) == 0 && ((q.ldc * c_esz) & 15) == 0 && ((q.m * c_esz) & 15) == 0) {
-      rc = make_map(&out->tmap_c, q.c, c_bf16 ? BBX_BF16 : BBX_F32, q.n, q.m, q.ldc, 32, 32, false);
+      rc = make_map(&out->tmap_c, q.c, c_bf16 ? BBX_BF16 : BBX_F32, q.n, q.m, q.ldc, 32, 32,
+                    CU_TENSOR_MAP_SWIZZLE_NONE);
       if (rc) return rc;
       out->flags |= EPI_TMA_STORE;
     }
@@ -380,15 +381,18 @@ static int build_problem(int in_dtype, const bbx_tc_problem_t& q, int bn_code, T
   }
   // C through TMA stores when its base, pitch and row length meet the 16-byte
   // rules and the epilogue does not read C: 32-row boxes of 64 bytes (16 f32 /
-  // 32 bf16), unswizzled, two per epilogue warp in turn. A TMA store clips the box at the tensor's edge in whole 16-byte
+  // 32 bf16), two per epilogue warp in turn. A TMA store clips the box at the tensor's edge in whole 16-byte
   // pieces of a row (measured: with m = 1031 f32 rows stored column-major,
   // element 1031 of a 16-byte piece holding 1028..1031 was written), so a row
   // length that is not a multiple of 16 bytes would write into the pitch
   // padding: such C goes through the staged stores.
   if (!(out->flags & EPI_BETA) && (((uintptr_t)q.c) & 15) == 0 && ((q.ldc * c_esz) & 15) == 0 &&
       ((q.n * c_esz) & 15) == 0) {
-    rc = make_map(&out->tmap_c, q.c, c_bf16 ? BBX_BF16 : BBX_F32, q.m, q.n, q.ldc, 64 / c_esz, 32, false);
+    const bool swizzle = c_bf16 || q.k <= kTcSwizzleF32MaxK;
+    rc = make_map(&out->tmap_c, q.c, c_bf16 ? BBX_BF16 : BBX_F32, q.m, q.n, q.ldc, 64 / c_esz, 32,
+                  swizzle ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
+    if (swizzle) out->flags |= EPI_SWIZZLE_C;
     out->flags |= EPI_TMA_STORE;
   }
   return BBX_OK;
@@ -429,7 +433,7 @@ using namespace bbx;
 struct bbx_tc_plan {
   int dtype = BBX_BF16;
   int bn = 256;
-  bool ep8 = false;  // eight epilogue warps (every problem's K <= kTcEp8MaxK, kTc2Ep8MaxK for the pair)
+  bool ep8 = false;  // eight epilogue warps (every problem's K <= kTcEp8MaxK, kTc2Ep8MaxK for the pair with f32 C)
   bool amn = false, bmn = true;
   int count = 0;
   int total_tiles = 0;
@@ -642,8 +646,12 @@ int bbx_tc_plan_create(int in_dtype, const bbx_tc_problem_t* problems, int count
   }
   p->total_tiles = tiles;
   int max_k = 0;
-  for (int i = 0; i < count; ++i) max_k = std::max(max_k, problems[i].k);
-  p->ep8 = max_k <= (tile_n == 512 ? kTc2Ep8MaxK : kTcEp8MaxK);
+  bool f32_c = true;
+  for (int i = 0; i < count; ++i) {
+    max_k = std::max(max_k, problems[i].k);
+    f32_c = f32_c && !(problems[i].flags & BBX_EPI_OUT_BF16);
+  }
+  p->ep8 = max_k <= (tile_n == 512 && f32_c ? kTc2Ep8MaxK : kTcEp8MaxK);
   if (count > kTcMaxInline) {
     cudaError_t e = cudaMalloc(&p->d_table, sizeof(TcProblem) * count);
     if (e != cudaSuccess) { delete p; return set_error(BBX_ERR_CUDA, "cudaMalloc(plan table): %s", cudaGetErrorString(e)); }

@@ -36,6 +36,7 @@ enum : int {
   EPI_BIAS = 4,      // add bias[col]
   EPI_BETA = 8,      // read C and add beta * C
   EPI_TMA_STORE = 16,  // set by the host: C is written by TMA stores through tmap_c
+  EPI_SWIZZLE_C = 64,  // set by the host: the row-major boxes of tmap_c are swizzled
   EPI_C_TRANS = 32,    // C is column-major: with EPI_TMA_STORE through tmap_c (boxes of 32 columns x 32
                        // rows of C), else by coalesced stores from registers
 };
@@ -44,8 +45,8 @@ enum : int {
 struct alignas(64) TcProblem {
   CUtensorMap tmap_a;  // 128 B
   CUtensorMap tmap_b;  // 128 B
-  CUtensorMap tmap_c;  // 128 B, valid with EPI_TMA_STORE: 32-row x 64-byte boxes (row-major C) or
-                       // 32 x 32-element boxes (column-major C), no swizzle
+  CUtensorMap tmap_c;  // 128 B, valid with EPI_TMA_STORE: 32-row x 64-byte boxes, 64-byte swizzle
+                       // (row-major C) or 32 x 32-element boxes, no swizzle (column-major C)
   void* c;
   const float* bias;
   long long ldc;       // elements
@@ -95,10 +96,14 @@ static_assert(32 * kTcEpiPitch * 4 <= kTcEpiSlot && 32 * 128 <= kTcEpiSlot && kT
 // blocks: 2609 -> 2453 TFLOP/s), so the host picks it only for short K.
 constexpr int kTcEp8MaxK = 512;
 // The same for the 2-SM pair kernel's 256 x 256 tiles: config 1's 64 x 1024^3
-// products 0.143 -> 0.128 ms. Not for longer K: with groups of K up to 2048 the
+// products 0.143 -> 0.128 ms with f32 C; with bf16 C (half the bytes to store)
+// only to kTcEp8MaxK: 64 x 1024^3 116 us with four warps, 123 with eight. Not for longer K: with groups of K up to 2048 the
 // 2000-op DAG's tensor groups ran 10 % faster alone but its makespan 2-4 %
 // slower, and the FFN step (K = 2048) 3 % slower.
 constexpr int kTc2Ep8MaxK = 1024;
+
+// Boxes of an f32 C whose K is above this are not swizzled (tc_epi_rows_tma).
+constexpr int kTcSwizzleF32MaxK = 512;
 
 template <int BN, bool A_MN, bool B_MN, bool FP8, bool EP8 = false>
 struct TcCfg {
@@ -334,7 +339,15 @@ __device__ __forceinline__ void tc_epi_rows(const TcProblem* pr, uint32_t t_row,
 // once the store issued from it has read it (cp.async.bulk.wait_group.read 1),
 // so filling one box overlaps the store of the other; with a single box each
 // 4 KB chunk waited for the previous store, which held the 2-SM headline
-// kernel at 0.87 of the burst peak (0.92 with two boxes, same box). `box_sel`
+// kernel at 0.87 of the burst peak (0.92 with two boxes, same box). The boxes
+// are swizzled (EPI_SWIZZLE_C): in plain 64-byte rows the eight lanes of a phase
+// of a 16-byte store hit two bank groups, and a 128 x 256 f32 tile takes 5500
+// cycles to leave an SM against 4400 (an SM writes 32 bytes a cycle, measured by any
+// kind of store: 4096). 60 x 512 x 512 x 256: 34.3 -> 28.9 us, 8 x 256^3 12.5 -> 10.5,
+// 16 x 2048^3 with bf16 C 230 -> 223. Not for f32 C behind a long main loop,
+// which has the shared memory busy all the time (32 KiB read and 32 KiB written per
+// 512 cycles of MMA): there the slower boxes disturb it less, 64 x 1024^3 137
+// against 141 us. `box_sel`
 // (per warp, kept across tiles) names the box to fill next; 2 means the last
 // store read the whole 4 KB slot (column-major C). With EPI_C_TRANS
 // (column-major C) the box is 32 columns x the warp's 32 rows, unswizzled, and
@@ -402,6 +415,7 @@ __device__ __forceinline__ void tc_epi_rows_tma(const TcProblem* pr, uint32_t t_
   // the other box's store may still be reading)
   (void)step;
   const int half = bf16 ? 32 : 16;
+  const int swz = (flags & EPI_SWIZZLE_C) ? (lane >> 1) & 3 : 0;
   if (box_sel == 2) {  // the last store read the whole 4 KB box (column-major C): let it finish
     if (lane == 0) bulk_wait_read_all();
     box_sel = 0;
@@ -459,8 +473,9 @@ __device__ __forceinline__ void tc_epi_rows_tma(const TcProblem* pr, uint32_t t_
     uint8_t* hb = box + box_sel * 2048;
     if (lane == 0) bulk_wait_read_1();
     __syncwarp();
+    // the map's 64-byte swizzle: piece j of row r lies at piece j ^ (r / 2 % 4)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) *(uint4*)(hb + lane * 64 + j * 16) = q[j];
+    for (int j = 0; j < 4; ++j) *(uint4*)(hb + lane * 64 + ((j ^ swz) << 4)) = q[j];
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {

@@ -63,7 +63,8 @@ def matmul_tc(problems, in_dtype=BF16, tile_n=0):
 
 
 # Groups whose largest K is at most this run with eight epilogue warps (the variant the
-# plan picks; `kTcEp8MaxK` / `kTc2Ep8MaxK` in csrc/gemm_tc.cuh): 1-SM tiles, the 2-SM pair.
+# plan picks; `kTcEp8MaxK` / `kTc2Ep8MaxK` in csrc/gemm_tc.cuh): 1-SM tiles and the 2-SM pair
+# with bf16 C, the 2-SM pair with f32 C.
 TC_EP8_MAX_K = 512
 TC2_EP8_MAX_K = 1024
 
@@ -77,6 +78,7 @@ class TcPlan:
         self.in_dtype = in_dtype
         self.trans = (bool(problems[0].trans_a), bool(problems[0].trans_b))
         self.max_k = max(int(p.k) for p in problems)
+        self.f32_c = not any(p.flags & EPI_OUT_BF16 for p in problems)
         check(lib.bbx_tc_plan_create(in_dtype, arr, len(problems), tile_n, C.byref(self.h)))
 
     def launch(self, stream=None):
@@ -93,7 +95,7 @@ class TcPlan:
         a = "MN-major A" if self.trans[0] else "K-major A"
         b = "K-major B" if self.trans[1] else "MN-major B"
         if tn == 512:
-            epi = "8 epilogue warps" if self.max_k <= TC2_EP8_MAX_K else "4 epilogue warps"
+            epi = "8 epilogue warps" if self.max_k <= (TC2_EP8_MAX_K if self.f32_c else TC_EP8_MAX_K) else "4 epilogue warps"
             return "tc_gemm2_kernel<%s,%s,%s> (2-SM 256x256 pair, cta_group::2)" % (a, b, epi)
         epi = "8 epilogue warps" if self.max_k <= TC_EP8_MAX_K else "4 epilogue warps"
         return "tc_gemm_kernel<%d,%s,%s,%s,%s>" % (tn, a, b, "e4m3" if self.in_dtype == E4M3 else "bf16", epi)
