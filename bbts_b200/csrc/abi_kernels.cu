@@ -88,10 +88,10 @@ static int set_tc_attrs() {
   return rc;
 }
 
-template <bool AMN, bool BMN, bool EP8>
+template <bool AMN, bool BMN, bool EP8, bool FP8 = false>
 static int set_tc2_attr() {
-  BBX_CUDA(cudaFuncSetAttribute(tc_gemm2_kernel<AMN, BMN, EP8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                Tc2Cfg<AMN, BMN, EP8>::SMEM_BYTES));
+  BBX_CUDA(cudaFuncSetAttribute(tc_gemm2_kernel<AMN, BMN, EP8, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                Tc2Cfg<AMN, BMN, EP8, FP8>::SMEM_BYTES));
   return BBX_OK;
 }
 
@@ -100,11 +100,21 @@ static int set_tc2_attrs() {
   int rc = 0;
   rc |= set_tc2_attr<false, false, EP8>(); rc |= set_tc2_attr<false, true, EP8>();
   rc |= set_tc2_attr<true, false, EP8>();  rc |= set_tc2_attr<true, true, EP8>();
+  rc |= set_tc2_attr<false, false, EP8, true>();
   return rc;
 }
 
-static int launch_tc2(bool amn, bool bmn, bool ep8, const TcArgs& args, int grid, cudaStream_t st) {
+static int launch_tc2(bool amn, bool bmn, bool fp8, bool ep8, const TcArgs& args, int grid, cudaStream_t st) {
   if (grid < 2) grid = 2;
+  if (fp8 && !amn && !bmn) {
+    using C4 = Tc2Cfg<false, false, false, true>;
+    using C8 = Tc2Cfg<false, false, true, true>;
+    if (ep8) tc_gemm2_kernel<false, false, true, true><<<grid, C8::THREADS, C8::SMEM_BYTES, st>>>(args);
+    else tc_gemm2_kernel<false, false, false, true><<<grid, C4::THREADS, C4::SMEM_BYTES, st>>>(args);
+    BBX_CHECK_LAUNCH("tc_gemm2_kernel");
+    return BBX_OK;
+  }
+  if (fp8) return set_error(BBX_ERR_UNSUPPORTED, "the e4m3 pair reads K-major operands");
 #define TC2_CASE(A_, B_, E_)                                                                  \
   if (amn == A_ && bmn == B_ && ep8 == E_) {                                                  \
     tc_gemm2_kernel<A_, B_, E_><<<grid, Tc2Cfg<A_, B_, E_>::THREADS, Tc2Cfg<A_, B_, E_>::SMEM_BYTES, st>>>(args); \
@@ -388,7 +398,7 @@ static int build_problem(int in_dtype, const bbx_tc_problem_t& q, int bn_code, T
   // padding: such C goes through the staged stores.
   if (!(out->flags & EPI_BETA) && (((uintptr_t)q.c) & 15) == 0 && ((q.ldc * c_esz) & 15) == 0 &&
       ((q.n * c_esz) & 15) == 0) {
-    const bool swizzle = c_bf16 || q.k <= kTcSwizzleF32MaxK;
+    const bool swizzle = c_bf16 || in_dtype == BBX_E4M3 || q.k <= kTcSwizzleF32MaxK;
     rc = make_map(&out->tmap_c, q.c, c_bf16 ? BBX_BF16 : BBX_F32, q.m, q.n, q.ldc, 64 / c_esz, 32,
                   swizzle ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
@@ -398,10 +408,11 @@ static int build_problem(int in_dtype, const bbx_tc_problem_t& q, int bn_code, T
   return BBX_OK;
 }
 
-// Default tile: the 2-SM 256 x 256 pair for bf16 groups whose problems are all
-// at least 256 x 256 and that fill every SM pair at least twice (measured
-// 6-7% above the 1-SM 128 x 256 tile on 4096^3 blocks); otherwise 128 x 256,
-// or 128 x 128 when no problem is wider than 128.
+// Default tile: the 2-SM 256 x 256 pair for bf16 groups, and e4m3 groups with
+// K-major operands and K >= kTc2Fp8MinK, whose problems are all at least 256 x 256 and that fill every
+// SM pair at least twice (measured 6-7% above the 1-SM 128 x 256 tile on 4096^3
+// bf16 blocks, 1.2 times on e4m3 ones); otherwise 128 x 256, or 128 x 128
+// when no problem is wider than 128.
 int pick_tile_n(const bbx_tc_problem_t* probs, int count, int in_dtype) {
   int maxn = 0, minmn = 1 << 30;
   long long pair_tiles = 0;
@@ -412,7 +423,13 @@ int pick_tile_n(const bbx_tc_problem_t* probs, int count, int in_dtype) {
   }
   DeviceState* d = nullptr;
   const int sms = device_state(&d) == BBX_OK ? d->sms : 148;
-  if (in_dtype == BBX_BF16 && minmn >= 256 && pair_tiles >= 2LL * (sms / 2)) return 512;
+  bool pair = in_dtype == BBX_BF16;
+  if (in_dtype == BBX_E4M3) {
+    pair = true;
+    for (int i = 0; i < count; ++i)
+      pair = pair && !probs[i].trans_a && probs[i].trans_b && probs[i].k >= kTc2Fp8MinK;  // K-major both
+  }
+  if (pair && minmn >= 256 && pair_tiles >= 2LL * (sms / 2)) return 512;
   return maxn > 128 ? 256 : 128;
 }
 
@@ -601,15 +618,17 @@ void f32_simt_plan_destroy(F32SimtPlan* p) { delete p; }
 
 extern "C" {
 
-int bbx_tc_plan_create(int in_dtype, const bbx_tc_problem_t* problems, int count, int tile_n,
-                       bbx_tc_plan_t** out) {
+// tile_n as the caller gave it, or as pick_tile_n chose it (by_rule).
+static int tc_plan_create(int in_dtype, const bbx_tc_problem_t* problems, int count, int tile_n, bool by_rule,
+                          bbx_tc_plan_t** out) {
   if (!out || !problems || count <= 0) return set_error(BBX_ERR_INVALID, "bad plan arguments");
   if (in_dtype != BBX_BF16 && in_dtype != BBX_E4M3)
     return set_error(BBX_ERR_UNSUPPORTED, "tensor-core input dtype must be bf16 or e4m3");
+  if (tile_n == 512 && in_dtype != BBX_BF16 && !by_rule)
+    return set_error(BBX_ERR_UNSUPPORTED, "the 2-SM tile of e4m3 operands is taken by the size rule only");
   if (tile_n == 0) tile_n = pick_tile_n(problems, count, in_dtype);
   if (tile_n != 128 && tile_n != 256 && tile_n != 512)
     return set_error(BBX_ERR_INVALID, "tile_n must be 128, 256 or 512 (2-SM 256x256 pair)");
-  if (tile_n == 512 && in_dtype != BBX_BF16) return set_error(BBX_ERR_UNSUPPORTED, "the 2-SM tile is bf16 only");
   DeviceState* d;
   int rc = device_state(&d);
   if (rc) return rc;
@@ -651,7 +670,7 @@ int bbx_tc_plan_create(int in_dtype, const bbx_tc_problem_t* problems, int count
     max_k = std::max(max_k, problems[i].k);
     f32_c = f32_c && !(problems[i].flags & BBX_EPI_OUT_BF16);
   }
-  p->ep8 = max_k <= (tile_n == 512 && f32_c ? kTc2Ep8MaxK : kTcEp8MaxK);
+  p->ep8 = max_k <= (in_dtype == BBX_E4M3 ? kTcFp8Ep8MaxK : tile_n == 512 && f32_c ? kTc2Ep8MaxK : kTcEp8MaxK);
   if (count > kTcMaxInline) {
     cudaError_t e = cudaMalloc(&p->d_table, sizeof(TcProblem) * count);
     if (e != cudaSuccess) { delete p; return set_error(BBX_ERR_CUDA, "cudaMalloc(plan table): %s", cudaGetErrorString(e)); }
@@ -660,6 +679,11 @@ int bbx_tc_plan_create(int in_dtype, const bbx_tc_problem_t* problems, int count
   }
   *out = p;
   return BBX_OK;
+}
+
+int bbx_tc_plan_create(int in_dtype, const bbx_tc_problem_t* problems, int count, int tile_n,
+                       bbx_tc_plan_t** out) {
+  return tc_plan_create(in_dtype, problems, count, tile_n, false, out);
 }
 
 int bbx_tc_plan_launch(bbx_tc_plan_t* p, void* stream) {
@@ -678,7 +702,7 @@ int bbx_tc_plan_launch(bbx_tc_plan_t* p, void* stream) {
   if (p->bn == 512) {
     // one CTA pair (cluster of 2) per 256 x 256 tile, persistent over the tile list
     const int grid = 2 * std::min(p->total_tiles, d->sms / 2);
-    return launch_tc2(p->amn, p->bmn, p->ep8, args, grid, (cudaStream_t)stream);
+    return launch_tc2(p->amn, p->bmn, p->dtype == BBX_E4M3, p->ep8, args, grid, (cudaStream_t)stream);
   }
   const int grid = std::min(p->total_tiles, d->sms);
   return launch_tc(p->bn, p->amn, p->bmn, p->dtype == BBX_E4M3, p->ep8, args, grid,
@@ -697,14 +721,15 @@ int bbx_tc_plan_destroy(bbx_tc_plan_t* p) {
 int bbx_matmul_tc(int in_dtype, const bbx_tc_problem_t* problems, int count, int tile_n,
                   void* stream) {
   if (count <= 0 || !problems) return set_error(BBX_ERR_INVALID, "no problems");
-  if (tile_n == 0) tile_n = pick_tile_n(problems, count, in_dtype);
+  const bool by_rule = tile_n == 0;
+  if (by_rule) tile_n = pick_tile_n(problems, count, in_dtype);
   // Problems travel in the kernel parameters, kTcMaxInline per launch: no
   // device table, no host-to-device copy, so the call is safe to capture in a
   // CUDA graph. Large groups that are launched repeatedly should use a plan.
   for (int i = 0; i < count; i += kTcMaxInline) {
     const int c = std::min(kTcMaxInline, count - i);
     bbx_tc_plan_t* p = nullptr;
-    int rc = bbx_tc_plan_create(in_dtype, problems + i, c, tile_n, &p);
+    int rc = tc_plan_create(in_dtype, problems + i, c, tile_n, by_rule, &p);
     if (rc) return rc;
     rc = bbx_tc_plan_launch(p, stream);
     bbx_tc_plan_destroy(p);  // inline plans own no device memory

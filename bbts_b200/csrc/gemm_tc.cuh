@@ -102,7 +102,13 @@ constexpr int kTcEp8MaxK = 512;
 // slower, and the FFN step (K = 2048) 3 % slower.
 constexpr int kTc2Ep8MaxK = 1024;
 
-// Boxes of an f32 C whose K is above this are not swizzled (tc_epi_rows_tma).
+// e4m3: both kernels. An e4m3 main loop is half as long as a bf16 one of the
+// same K, so the epilogue sets the pace further: 16 x 1040^3 80.5 -> 64.5 us (1-SM),
+// 16 x 2048^3 143 -> 133 (pair). The pair pays from kTc2Fp8MinK on: 4 x 4096^3 253 ->
+// 208 us against the 1-SM tile, 20 x 512 x 2048 x 512 28 against 47 the other way.
+constexpr int kTcFp8Ep8MaxK = 2048;
+constexpr int kTc2Fp8MinK = 1536;
+// Boxes of a bf16 product's f32 C whose K is above this are not swizzled (tc_epi_rows_tma).
 constexpr int kTcSwizzleF32MaxK = 512;
 
 template <int BN, bool A_MN, bool B_MN, bool FP8, bool EP8 = false>
@@ -692,14 +698,18 @@ __global__ void __launch_bounds__(EP8 ? 320 : 192, 1) tc_gemm_kernel(const __gri
 // full barrier; the leader's single MMA thread commits each stage back to the
 // empty barriers of both CTAs and each accumulator to both CTAs' tfull
 // barriers; both epilogues release the accumulator on the leader's tempty.
-// bf16 only.
+// bf16 operands of either major-ness, or e4m3 ones that are both K-major (the
+// layout that the quantisation writes). The e4m3 1-SM 128 x 256 tile needs 48 KiB
+// read and 48 KiB written in shared memory per 512 cycles of MMA, 1.5 times what
+// there is; the pair needs 32 + 32.
 // ============================================================================
-template <bool A_MN, bool B_MN, bool EP8 = false>
+template <bool A_MN, bool B_MN, bool EP8 = false, bool FP8 = false>
 struct Tc2Cfg {
+  static_assert(!FP8 || (!A_MN && !B_MN), "the e4m3 pair reads K-major operands");
   static constexpr int BM = 256;  // rows per pair (128 per CTA)
   static constexpr int BN = 256;  // columns per pair (128 B rows per CTA)
-  static constexpr int BK = 64;
-  static constexpr int UMMA_K = 16;
+  static constexpr int BK = FP8 ? 128 : 64;  // one 128-byte swizzle row of K
+  static constexpr int UMMA_K = FP8 ? 32 : 16;
   static constexpr int A_BYTES = 128 * 128;  // 128 rows x 128 B
   static constexpr int B_BYTES = 128 * 128;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -713,10 +723,10 @@ struct Tc2Cfg {
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
 };
 
-template <bool A_MN, bool B_MN, bool EP8>
+template <bool A_MN, bool B_MN, bool EP8, bool FP8 = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EP8 ? 320 : 192, 1)
     tc_gemm2_kernel(const __grid_constant__ TcArgs args) {
-  using C = Tc2Cfg<A_MN, B_MN, EP8>;
+  using C = Tc2Cfg<A_MN, B_MN, EP8, FP8>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* stage_base = smem;
@@ -823,7 +833,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EP8 ? 320 : 192, 1)
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     if (leader && lane == 0) {
-      constexpr uint32_t idesc = make_idesc(256, 256, 1u, A_MN, B_MN);
+      constexpr uint32_t idesc = make_idesc(256, 256, FP8 ? 0u : 1u /* e4m3 / bf16 */, A_MN, B_MN);
       int s = 0;
       uint32_t ph = 0;
       int acc = 0;
@@ -849,7 +859,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EP8 ? 320 : 192, 1)
             else da = smem_desc_sw128(sa + kk * (C::UMMA_K * 128), C::BK * 128, 1024);
             if constexpr (!B_MN) db = smem_desc_sw128(sb + kk * 32, 16, 1024);
             else db = smem_desc_sw128(sb + kk * (C::UMMA_K * 128), C::BK * 128, 1024);
-            umma_f16_2sm(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            if constexpr (FP8) umma_f8_2sm(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            else umma_f16_2sm(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit_2sm(&empty_bar[s], 0x3);
           if (++s == C::STAGES) { s = 0; ph ^= 1; }

@@ -293,7 +293,7 @@ int autotune_tile_n(int dtype, bool ta, bool tb, const std::vector<bbx_tc_proble
   // so no plan's table lands where another candidate's tensor maps were used
   std::vector<std::pair<int, bbx_tc_plan_t*>> cand;
   for (int tn : {512, 256, 128}) {
-    if (tn == 512 && dtype == ELEM_E4M3) continue;  // the 2-SM pair tile is bf16 only
+    if (tn == 512 && dtype == ELEM_E4M3) continue;  // the e4m3 pair is for the size rule only
     bbx_tc_plan_t* p = nullptr;
     if (bbx_tc_plan_create(dtype == ELEM_E4M3 ? BBX_E4M3 : BBX_BF16, ps.data(), (int)ps.size(), tn, &p) == 0)
       cand.push_back({tn, p});

@@ -341,6 +341,17 @@ __device__ __forceinline__ void umma_f16_2sm(uint32_t d_tmem, uint64_t a_desc, u
       : "memory");
 }
 
+// The same for kind::f8f6f4.
+__device__ __forceinline__ void umma_f8_2sm(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // Pair form of umma_f16_shift_d.
 template <int SHIFT>
 __device__ __forceinline__ void umma_f16_2sm_shift_d(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,

@@ -67,6 +67,7 @@ def matmul_tc(problems, in_dtype=BF16, tile_n=0):
 # with bf16 C, the 2-SM pair with f32 C.
 TC_EP8_MAX_K = 512
 TC2_EP8_MAX_K = 1024
+FP8_EP8_MAX_K = 2048  # e4m3, either tile
 
 
 class TcPlan:
@@ -95,9 +96,12 @@ class TcPlan:
         a = "MN-major A" if self.trans[0] else "K-major A"
         b = "K-major B" if self.trans[1] else "MN-major B"
         if tn == 512:
-            epi = "8 epilogue warps" if self.max_k <= (TC2_EP8_MAX_K if self.f32_c else TC_EP8_MAX_K) else "4 epilogue warps"
-            return "tc_gemm2_kernel<%s,%s,%s> (2-SM 256x256 pair, cta_group::2)" % (a, b, epi)
-        epi = "8 epilogue warps" if self.max_k <= TC_EP8_MAX_K else "4 epilogue warps"
+            most = FP8_EP8_MAX_K if self.in_dtype == E4M3 else TC2_EP8_MAX_K if self.f32_c else TC_EP8_MAX_K
+            epi = "8 epilogue warps" if self.max_k <= most else "4 epilogue warps"
+            dt = "e4m3," if self.in_dtype == E4M3 else ""
+            return "tc_gemm2_kernel<%s,%s,%s%s> (2-SM 256x256 pair, cta_group::2)" % (a, b, dt, epi)
+        most = FP8_EP8_MAX_K if self.in_dtype == E4M3 else TC_EP8_MAX_K
+        epi = "8 epilogue warps" if self.max_k <= most else "4 epilogue warps"
         return "tc_gemm_kernel<%d,%s,%s,%s,%s>" % (tn, a, b, "e4m3" if self.in_dtype == E4M3 else "bf16", epi)
 
     def close(self):
