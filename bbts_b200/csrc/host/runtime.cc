@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cerrno>
+#include <chrono>
 #include <cstring>
 #include <cmath>
 #include <numeric>
@@ -890,16 +891,31 @@ void runtime_t::run_per_op(int policy, std::vector<std::pair<op_features_t, floa
       feats.push_back(features(*cmd, &hint));
       cudaEventCreate(&e0);
       cudaEventCreate(&e1);
-      cudaEventRecord(e0, s);
     }
-    storage->begin_command();
-    try {
-      execute_command(*this, *cmd, s, keep_chain.count(cmd->id) != 0);
-    } catch (...) {
+    // A host thread held up between the two events (another process on its core,
+    // memory being mapped) leaves the device idle inside the bracket: a command
+    // that kept the host longer than any launch takes, and whose measured time is
+    // mostly that, is timed again. Commands are functions of their inputs, uniform aside.
+    for (int attempt = 0;; ++attempt) {
+      const auto h0 = std::chrono::steady_clock::now();
+      if (record) cudaEventRecord(e0, s);
+      storage->begin_command();
+      try {
+        execute_command(*this, *cmd, s, keep_chain.count(cmd->id) != 0);
+      } catch (...) {
+        storage->end_command(s);
+        throw;
+      }
       storage->end_command(s);
-      throw;
+      if (!record) break;
+      cudaEventRecord(e1, s);
+      const double host_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - h0).count();
+      if (host_us < 150.0 || attempt == 2 || cmd->get_num_inputs() == 0) break;
+      cuda_ok(cudaEventSynchronize(e1), "record sync");
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e0, e1);
+      if (ms * 1000.f < 0.5 * host_us) break;  // the launch queue was full: the device was busy
     }
-    storage->end_command(s);
     if (hint_readers) {
       for (size_t j = 0; j < cmd->get_num_inputs(); ++j) {
         const tid_t t = cmd->get_input(j).tid;
@@ -911,10 +927,7 @@ void runtime_t::run_per_op(int policy, std::vector<std::pair<op_features_t, floa
         storage->set_readers_left(t, r == readers_left.end() ? 0 : r->second);
       }
     }
-    if (record) {
-      cudaEventRecord(e1, s);
-      evs.push_back({e0, e1});
-    }
+    if (record) evs.push_back({e0, e1});
     if (K > 1) {
       cudaEvent_t done = new_event();
       cuda_ok(cudaEventRecord(done, s), "record done");
