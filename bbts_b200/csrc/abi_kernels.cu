@@ -15,6 +15,7 @@
 #include "contraction.h"
 #include "f32tc.h"
 #include "gemm_f32.cuh"
+#include "launch.h"
 #include "gemm_tc.cuh"
 #include "stream_ops.cuh"
 
@@ -109,15 +110,16 @@ static int launch_tc2(bool amn, bool bmn, bool fp8, bool ep8, const TcArgs& args
   if (fp8 && !amn && !bmn) {
     using C4 = Tc2Cfg<false, false, false, true>;
     using C8 = Tc2Cfg<false, false, true, true>;
-    if (ep8) tc_gemm2_kernel<false, false, true, true><<<grid, C8::THREADS, C8::SMEM_BYTES, st>>>(args);
-    else tc_gemm2_kernel<false, false, false, true><<<grid, C4::THREADS, C4::SMEM_BYTES, st>>>(args);
+    if (ep8) launch_dependent(tc_gemm2_kernel<false, false, true, true>, grid, C8::THREADS, C8::SMEM_BYTES, st, args);
+    else launch_dependent(tc_gemm2_kernel<false, false, false, true>, grid, C4::THREADS, C4::SMEM_BYTES, st, args);
     BBX_CHECK_LAUNCH("tc_gemm2_kernel");
     return BBX_OK;
   }
   if (fp8) return set_error(BBX_ERR_UNSUPPORTED, "the e4m3 pair reads K-major operands");
 #define TC2_CASE(A_, B_, E_)                                                                  \
   if (amn == A_ && bmn == B_ && ep8 == E_) {                                                  \
-    tc_gemm2_kernel<A_, B_, E_><<<grid, Tc2Cfg<A_, B_, E_>::THREADS, Tc2Cfg<A_, B_, E_>::SMEM_BYTES, st>>>(args); \
+    launch_dependent(tc_gemm2_kernel<A_, B_, E_>, grid, Tc2Cfg<A_, B_, E_>::THREADS,                    \
+                     Tc2Cfg<A_, B_, E_>::SMEM_BYTES, st, args);                                         \
     BBX_CHECK_LAUNCH("tc_gemm2_kernel");                                                      \
     return BBX_OK;                                                                            \
   }
@@ -290,7 +292,7 @@ static int launch_tc_variant(const TcArgs& args, int grid, cudaStream_t st, Devi
     BBX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     d->attr_done |= (1u << bit);
   }
-  kern<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(args);
+  launch_dependent(kern, grid, C::THREADS, C::SMEM_BYTES, st, args);
   BBX_CHECK_LAUNCH("tc_gemm_kernel");
   return BBX_OK;
 }
@@ -791,8 +793,7 @@ int bbx_reduce_f32(const float* const* inputs, int n_in, float* out, long long n
       continue;
     }
     const int grid = grid_for((n + 3) / 4, 256, d->sms);
-    if (kahan) k_reduce<true><<<grid, 256, 0, st>>>(ra, cnt, out, n);
-    else k_reduce<false><<<grid, 256, 0, st>>>(ra, cnt, out, n);
+    launch_dependent(kahan ? k_reduce<true> : k_reduce<false>, grid, 256, 0, st, ra, cnt, out, n);
     BBX_CHECK_LAUNCH("k_reduce");
   }
   return BBX_OK;
@@ -1092,13 +1093,13 @@ int bbx_stream_plan_launch(bbx_stream_plan_t* p, void* stream) {
   if (rc) return rc;
   if (p->bulk) {
     const long long grid = std::min<long long>(p->total_chunks, (long long)d->sms);
-    k_stream_bulk<kBulkStoreTS><<<(int)grid, kBulkThreads, bulk_smem_bytes(p->count), (cudaStream_t)stream>>>(
+    launch_dependent(k_stream_bulk<kBulkStoreTS>, (int)grid, kBulkThreads, bulk_smem_bytes(p->count), (cudaStream_t)stream,
         p->d_table, p->count, p->total_chunks, d->status, kBulkPiece);
     BBX_CHECK_LAUNCH("k_stream_bulk");
     return BBX_OK;
   }
   long long grid = std::min<long long>(p->total_chunks, (long long)d->sms * 8);
-  k_stream_group<<<(int)grid, 256, 0, (cudaStream_t)stream>>>(p->d_table, p->count, p->total_chunks);
+  launch_dependent(k_stream_group, (int)grid, 256, 0, (cudaStream_t)stream, p->d_table, p->count, p->total_chunks);
   BBX_CHECK_LAUNCH("k_stream_group");
   return BBX_OK;
 }
@@ -1134,13 +1135,13 @@ int bbx_stream_group(const bbx_stream_op_t* ops, int count, void* stream) {
     for (int j = 0; j < c; ++j) args.ops[j] = table[j];
     if (bulk) {
       const long long grid = std::min<long long>(total, (long long)d->sms);
-      k_stream_bulk_inline<kBulkStoreTS><<<(int)grid, kBulkThreads, bulk_smem_bytes(c), (cudaStream_t)stream>>>(
+      launch_dependent(k_stream_bulk_inline<kBulkStoreTS>, (int)grid, kBulkThreads, bulk_smem_bytes(c), (cudaStream_t)stream,
           args, c, total, d->status, kBulkPiece);
       BBX_CHECK_LAUNCH("k_stream_bulk_inline");
       continue;
     }
     long long grid = std::min<long long>(total, (long long)d->sms * 8);
-    k_stream_group_inline<<<(int)grid, 256, 0, (cudaStream_t)stream>>>(args, c, total);
+    launch_dependent(k_stream_group_inline, (int)grid, 256, 0, (cudaStream_t)stream, args, c, total);
     BBX_CHECK_LAUNCH("k_stream_group_inline");
   }
   return BBX_OK;

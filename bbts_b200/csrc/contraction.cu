@@ -26,6 +26,7 @@
 #include "common.h"
 #include "contraction.h"
 #include "f32tc.h"
+#include "launch.h"
 #include "ptx.cuh"
 
 namespace bbx {
@@ -61,6 +62,8 @@ __device__ __forceinline__ void gather_one(const float* __restrict__ in, void* o
 
 __global__ void k_gather_sum(const float* __restrict__ in, void* out, int out_bf16,
                              const __grid_constant__ GatherArgs a, long long n) {
+  griddep_launch();
+  griddep_wait();
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
        e += (long long)gridDim.x * blockDim.x)
     gather_one(in, out, out_bf16, a, e);
@@ -187,6 +190,8 @@ __device__ __forceinline__ void gather_rows(const GatherRec& rec, long long item
 
 // One gather record on the row path (the per-call contraction).
 __global__ void k_gather_rows1(const __grid_constant__ GatherRec r, long long chunks) {
+  griddep_launch();
+  griddep_wait();
   const long long items = (r.n / r.row_len) * r.segs;
   for (long long c = blockIdx.x; c < chunks; c += gridDim.x) {
     const long long i0 = c * r.items_per_chunk;
@@ -201,6 +206,8 @@ __global__ void k_gather_rows1(const __grid_constant__ GatherRec r, long long ch
 // registers, a few spilled): the row loop's loads are latency-bound, and the
 // 2000-op DAG's input gathers went 0.83 -> 0.59 ms against three CTAs at 80.
 __global__ void __launch_bounds__(256, 4) k_gather_group(const GatherRec* __restrict__ recs, int count, long long total_chunks) {
+  griddep_launch();
+  griddep_wait();
   int lo = -1;
   for (long long c = blockIdx.x; c < total_chunks; c += gridDim.x) {
     if (lo < 0) {
@@ -272,6 +279,8 @@ __global__ void __launch_bounds__(kGBThreads, 1) k_gather_bulk(const GatherRec* 
     fence_mbar_init();
   }
   for (int i = threadIdx.x; i < count; i += blockDim.x) starts[i] = recs[i].chunk_start;
+  griddep_launch();
+  griddep_wait();
   __syncthreads();
   volatile uint32_t* st = status;
   const long long step = (long long)gridDim.x * kGBItems;
@@ -382,14 +391,14 @@ static int launch_gather(const float* in, void* out, bool bf16, const GatherArgs
     r.n = n;
     set_row_mode(&r);
     const long long chunks = (row_items(r) + r.items_per_chunk - 1) / r.items_per_chunk;
-    k_gather_rows1<<<(int)std::min<long long>(chunks, 148 * 8), 256, 0, st>>>(r, chunks);
+    launch_dependent(k_gather_rows1, (int)std::min<long long>(chunks, 148 * 8), 256, 0, st, r, chunks);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(BBX_ERR_CUDA, "k_gather_rows1: %s", cudaGetErrorString(e));
     return BBX_OK;
   }
   long long blocks = (n + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  k_gather_sum<<<(int)blocks, 256, 0, st>>>(in, out, bf16 ? 1 : 0, a, n);
+  launch_dependent(k_gather_sum, (int)blocks, 256, 0, st, in, out, bf16 ? 1 : 0, a, n);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(BBX_ERR_CUDA, "k_gather_sum: %s", cudaGetErrorString(e));
   return BBX_OK;
@@ -628,14 +637,14 @@ int gather_plan_launch(GatherPlan* p, void* stream) {
     int rc = device_status_and_sms(&status, &sms);
     if (rc) return rc;
     const long long grid = std::min<long long>((p->total + kGBItems - 1) / kGBItems, sms);
-    k_gather_bulk<<<(int)grid, kGBThreads, gb_smem_bytes(p->count), (cudaStream_t)stream>>>(p->d, p->count,
-                                                                                          p->total, status);
+    launch_dependent(k_gather_bulk, (int)grid, kGBThreads, gb_smem_bytes(p->count), (cudaStream_t)stream, p->d, p->count,
+                     p->total, status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(BBX_ERR_CUDA, "k_gather_bulk: %s", cudaGetErrorString(e));
     return BBX_OK;
   }
   long long grid = std::min<long long>(p->total, 148 * 8);
-  k_gather_group<<<(int)grid, 256, 0, (cudaStream_t)stream>>>(p->d, p->count, p->total);
+  launch_dependent(k_gather_group, (int)grid, 256, 0, (cudaStream_t)stream, p->d, p->count, p->total);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(BBX_ERR_CUDA, "k_gather_group: %s", cudaGetErrorString(e));
   return BBX_OK;

@@ -9,6 +9,7 @@
 #include "common.h"
 #include "f32tc.h"
 #include "gemm_f32tc.cuh"
+#include "launch.h"
 
 namespace bbx {
 
@@ -230,8 +231,7 @@ Shape pick_shape(const F3Mat* mats, const F3Spec* specs, const int* order, int c
 
 int launch(const F3Args& args, Shape shape, int sms, cudaStream_t st) {
   const int grid = kShapes[shape].sms * std::min(args.total_tiles, sms / kShapes[shape].sms);
-  if (shape == PAIR256) f32_gemm_pair_kernel<<<grid, kF3Threads, kF3Smem, st>>>(args);
-  else f32_gemm_kernel<<<grid, kF3Threads, kF3Smem, st>>>(args);
+  launch_dependent(shape == PAIR256 ? f32_gemm_pair_kernel : f32_gemm_kernel, grid, kF3Threads, kF3Smem, st, args);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? BBX_OK : set_error(BBX_ERR_CUDA, "f32_gemm: %s", cudaGetErrorString(e));
 }
@@ -252,9 +252,7 @@ SplitKind split_kind(const F3Split& r) {
 
 int launch_split(const F3SplitArgs& args, int chunks, int kind, cudaStream_t st) {
   if (chunks == 0) return BBX_OK;
-  if (kind == FLAT) k_f32_split_flat<<<chunks, 256, 0, st>>>(args);
-  else if (kind == ROWS) k_f32_split_rows<<<chunks, 256, 0, st>>>(args);
-  else k_f32_split<<<chunks, 256, 0, st>>>(args);
+  launch_dependent(kind == FLAT ? k_f32_split_flat : kind == ROWS ? k_f32_split_rows : k_f32_split, chunks, 256, 0, st, args);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? BBX_OK : set_error(BBX_ERR_CUDA, "k_f32_split: %s", cudaGetErrorString(e));
 }

@@ -207,6 +207,7 @@ __device__ __forceinline__ const F3Split& f3_split_record(const F3SplitArgs& arg
 // in flight, 16-byte accesses, few registers so that 48 warps fit an SM. The general form
 // below moved the same records at 2.5 TB/s (64-bit index arithmetic, 80 registers).
 __global__ void __launch_bounds__(256, 6) k_f32_split_flat(const __grid_constant__ F3SplitArgs args) {
+  griddep_launch();
   const F3Split& r = f3_split_record(args, blockIdx.x);
   const float* __restrict__ src = r.src;
   __nv_bfloat16* const dst = r.dst;
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(256, 6) k_f32_split_flat(const __grid_constant
   uint4* const dp = (uint4*)dst + i0;
   const long long pw = plane / 8;
   uint32_t mx = 0;
+  griddep_wait();
   for (int it = threadIdx.x; it < n; it += 512) {
     const bool two = it + 256 < n;
     const float4 a = __ldg(sp + 2 * it), b = __ldg(sp + 2 * it + 1);
@@ -246,6 +248,7 @@ __global__ void __launch_bounds__(256, 6) k_f32_split_flat(const __grid_constant
 // contraction's operands moved at 1.7 TB/s), except at the ends of the tensor,
 // where a piece could reach outside it.
 __global__ void __launch_bounds__(256, 5) k_f32_split_rows(const __grid_constant__ F3SplitArgs args) {
+  griddep_launch();
   const F3Split& r = f3_split_record(args, blockIdx.x);
   const float* __restrict__ src = r.src;
   __nv_bfloat16* const dst = r.dst;
@@ -256,6 +259,7 @@ __global__ void __launch_bounds__(256, 5) k_f32_split_rows(const __grid_constant
   const uint32_t i1 = (uint32_t)min((long long)i0 + r.items_per_chunk, r.items);
   const float* const last = src + (r.odims[2] - 1) * istr + len;  // one past the tensor
   uint32_t mx = 0;
+  griddep_wait();
   for (uint32_t it = i0 + threadIdx.x; it < i1; it += 256) {
     const uint32_t row = it / per_row, e = (it - row * per_row) * 8;
     const int cnt = (int)min(8u, len - e);
@@ -288,6 +292,7 @@ __global__ void __launch_bounds__(256, 5) k_f32_split_rows(const __grid_constant
 
 // Any record: strided rows, gathers, summed modes, unaligned rows.
 __global__ void __launch_bounds__(256) k_f32_split(const __grid_constant__ F3SplitArgs args) {
+  griddep_launch();
   const int chunk = blockIdx.x;
   const F3Split& r = f3_split_record(args, chunk);
   const float* __restrict__ src = r.src;
@@ -301,6 +306,7 @@ __global__ void __launch_bounds__(256) k_f32_split(const __grid_constant__ F3Spl
   const long long os0 = r.ostride[0], os1 = r.ostride[1], os2 = r.ostride[2];
   const bool small = r.items < (1ll << 31) && od1 * od2 < (1ll << 31);
   uint32_t mx = 0;
+  griddep_wait();
   for (long long it = i0 + threadIdx.x; it < i1; it += blockDim.x) {
     long long row, c8;
     if (small) {  // 32-bit division
@@ -590,7 +596,10 @@ __device__ __forceinline__ void f3_gemm_body(const F3Args& args) {
   } else if (warp == 1) {
     if constexpr (PAIR) tmem_alloc_2sm(tmem_slot, TMEM_COLS);
     else tmem_alloc(tmem_slot, TMEM_COLS);
-  } else {
+  }
+  griddep_launch();
+  griddep_wait();  // the maxima below are the split's
+  if (warp >= 2) {
     // one warp per problem: its tiles, and whether its operands are in range
     for (int p = warp - 2; p < args.num_problems; p += kF3EpiWarps) {
       const F3Fields f = f3_fields(args, p);

@@ -534,6 +534,8 @@ __global__ void __launch_bounds__(EP8 ? 320 : 192, 1) tc_gemm_kernel(const __gri
   }
   tc_stage_meta(args, meta);
   if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
+  griddep_launch();
+  griddep_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -762,6 +764,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EP8 ? 320 : 192, 1)
   }
   tc_stage_meta(args, meta);
   if (warp == 1) tmem_alloc_2sm(tmem_slot, C::TMEM_COLS);
+  griddep_launch();
+  griddep_wait();
   tc_fence_before();
   __syncthreads();
   __syncwarp();

@@ -42,6 +42,7 @@
 #include <string>
 #include "contraction.h"
 #include "f32tc.h"
+#include "launch.h"
 #include "runtime.h"
 
 namespace bbx {
@@ -1043,10 +1044,18 @@ static dag_t* dag_build_as(runtime_t* rt, int policy, int tile_n, bool f32_tc, b
     dag_cuda(cudaEventRecord(fork, origin), "fork");
     dag_cuda(cudaStreamWaitEvent(s_mem, fork, 0), "fork mem");
     dag_cuda(cudaStreamWaitEvent(s_tc, fork, 0), "fork tc");
+    // A group that is alone in its wave, behind a wave of one group, follows it
+    // on that group's stream: the two cannot overlap, and on one stream the second's
+    // prologue overlaps the first's tail (programmatic dependent launch).
+    std::vector<int> in_wave(nw, 0);
+    for (const group_t& g : d->groups) ++in_wave[g.wave];
     std::vector<bool> on_tc(d->groups.size());
     for (size_t gi = 0; gi < d->groups.size(); ++gi) {
       group_t& g = d->groups[gi];
       on_tc[gi] = g.kind == G_TC;
+      if (gi > 0 && in_wave[g.wave] == 1 && d->groups[gi - 1].wave == g.wave - 1 && in_wave[g.wave - 1] == 1)
+        on_tc[gi] = on_tc[gi - 1];
+      const bbx::PlainLaunches plain(in_wave[g.wave] > 1);
       cudaStream_t st = on_tc[gi] ? s_tc : s_mem;
       for (int dep : g.deps)
         if (on_tc[dep] != on_tc[gi]) dag_cuda(cudaStreamWaitEvent(st, ev[dep], 0), "dependency");

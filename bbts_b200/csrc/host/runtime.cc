@@ -1,6 +1,7 @@
 // Runtime: block storage, per-op runner and the grouped DAG executor.
 #include "runtime.h"
 #include "f32tc.h"
+#include "launch.h"
 
 #include <fcntl.h>
 #include <unistd.h>
@@ -790,6 +791,7 @@ void runtime_t::run_per_op(int policy, std::vector<std::pair<op_features_t, floa
 
   // ---- worker streams (one = the runtime stream itself)
   const int K = record ? 1 : std::max(1, std::min(workers, 16));
+  const bbx::PlainLaunches plain(K > 1);
   while ((int)worker_streams.size() < K && K > 1) {
     cudaStream_t s;
     cuda_ok(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate(worker)");

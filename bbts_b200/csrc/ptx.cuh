@@ -45,6 +45,17 @@ __device__ __forceinline__ bool elect_one() {
 // Lane 0's value in every lane (warp-uniform).
 __device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 
+// Programmatic dependent launch (launch_dependent in launch.h). griddep_launch
+// lets the next kernel of the stream start its own prologue as soon as every
+// block of this one runs (or has exited); griddep_wait returns when the kernels
+// before this one have completed and their writes are visible. Every thread of
+// a kernel that is launched this way runs griddep_wait before it touches memory
+// that an earlier kernel may write or read; before it, only parameters and plan
+// tables (uploaded when the plan was made) are read. A kernel is held back by its
+// predecessor's predecessors too: the predecessor cannot complete before them.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

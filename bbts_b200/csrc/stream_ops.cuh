@@ -164,6 +164,8 @@ __global__ void k_binary(int op, const float* a, const float* b, float* c, long 
 template <bool KAHAN>
 __global__ void k_reduce(const __grid_constant__ ReduceArgs args, int n_in, float* out,
                          long long n) {
+  griddep_launch();
+  griddep_wait();
   long long i4 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   bool vec = (((uintptr_t)out) & 15) == 0;
@@ -617,6 +619,8 @@ __global__ void __launch_bounds__(256) k_stream_group_inline(const __grid_consta
 template <typename TableT>
 __device__ __forceinline__ void stream_group_body(const TableT* __restrict__ table, int count,
                                                   long long total_chunks) {
+  griddep_launch();
+  griddep_wait();
   for (long long c = blockIdx.x; c < total_chunks; c += gridDim.x) {
     int lo = 0, hi = count - 1;
     while (lo < hi) {
@@ -915,6 +919,8 @@ __device__ __forceinline__ void stream_bulk_body(const TableT* table, int count,
   }
   if (staged)
     for (int i = threadIdx.x; i < count; i += blockDim.x) starts[i] = table[i].chunk_start;
+  griddep_launch();
+  griddep_wait();
   __syncthreads();
   volatile uint32_t* st = status;
   if (warp == kBulkConsumerWarps) {
