@@ -65,7 +65,9 @@ struct GatherRec {
   long long chunk_start;   // set by gather_plan_create
   long long row_len;       // row mode: elements per row (the innermost extent, after merging)
   long long segs;          // row mode: segments of kGatherSeg elements per row
-  long long items_per_chunk;  // row mode: (row, segment) items per chunk
+  long long items_per_chunk;  // row mode: (row, segment) items per chunk; wide: pieces per chunk
+  int wide;                // row mode, 16-byte aligned destination rows: pieces of eight elements
+  long long src_elems;     // wide: elements of the source from src to the last one read
 };
 
 // Elements per work item of the row path: one segment of a row.
