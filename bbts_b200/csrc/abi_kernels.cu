@@ -378,17 +378,9 @@ static int build_problem(int in_dtype, const bbx_tc_problem_t& q, int bn_code, T
   const bool c_bf16 = (out->flags & EPI_OUT_BF16) != 0;
   const int c_esz = c_bf16 ? 2 : 4;
   if (c_col) {
-    // column-major C: stored n rows of m. With the 16-byte rules met, each
-    // epilogue warp stores its 32 rows of C as TMA boxes of 32 columns x 32
-    // m-elements (no swizzle); otherwise by coalesced stores from registers.
+    // column-major C: coalesced stores from registers, whatever its alignment
     if (out->flags & EPI_BETA) return set_error(BBX_ERR_UNSUPPORTED, "column-major C with beta");
     out->flags |= EPI_C_TRANS;
-    if ((((uintptr_t)q.c) & 15) == 0 && ((q.ldc * c_esz) & 15) == 0 && ((q.m * c_esz) & 15) == 0) {
-      rc = make_map(&out->tmap_c, q.c, c_bf16 ? BBX_BF16 : BBX_F32, q.n, q.m, q.ldc, 32, 32,
-                    CU_TENSOR_MAP_SWIZZLE_NONE);
-      if (rc) return rc;
-      out->flags |= EPI_TMA_STORE;
-    }
     return BBX_OK;
   }
   // C through TMA stores when its base, pitch and row length meet the 16-byte

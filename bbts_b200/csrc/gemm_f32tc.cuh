@@ -478,11 +478,20 @@ template <int NC>
 __device__ __forceinline__ void f3_store(const F3Out& o, int row0, int col0, int lane, float* stage, const float (&acc)[NC]) {
   if (row0 >= o.m) return;
   if (o.c_col) {
-    const bool row_ok = row0 + lane < o.m;
+    if (row0 + lane >= o.m) return;
     float* cp = o.c + row0 + lane + (long long)col0 * o.ldc;
 #pragma unroll
-    for (int j = 0; j < NC; ++j, cp += o.ldc)
-      if (col0 + j < o.n && row_ok) *cp = f3_finish(o, acc[j], cp, col0 + j);
+    for (int j0 = 0; j0 < NC; j0 += 32) {
+      const int left = o.n - col0 - j0;
+      if (left >= 32 && o.plain) {  // no test per column
+#pragma unroll
+        for (int j = 0; j < 32; ++j, cp += o.ldc) *cp = o.alpha * acc[j0 + j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j, cp += o.ldc)
+          if (j < left) *cp = f3_finish(o, acc[j0 + j], cp, col0 + j0 + j);
+      }
+    }
     return;
   }
   const bool vec = ((((uintptr_t)o.c) & 15) == 0) && (o.ldc & 3) == 0 && (o.n & 3) == 0;
