@@ -91,8 +91,10 @@ int bbx_num_sms(void);
 int bbx_check_device_status(void* stream, uint32_t* code_out);
 
 /* ------------------------------------------------------------------ block matmul */
-/* FP32 SIMT matmul: C = alpha*op(A)*op(B) + beta*C (+bias[col]) (relu), batched
- * over `batch` with element strides. Replaces dense_matrix_mult_t::mult
+/* FP32 matmul: C = alpha*op(A)*op(B) + beta*C (+bias[col]) (relu), batched
+ * over `batch` with element strides. Large products run on the tensor cores (each
+ * operand split into three bf16 planes in stream-ordered scratch; FP32 accuracy),
+ * small ones, and all under stream capture, on a SIMT kernel. Replaces dense_matrix_mult_t::mult
  * (dense_matrix_mult.cc:78-82: cblas_sgemm RowMajor with trans flags b0/b1) and
  * the batched cblas_sgemm_batch_strided of contraction.h:439-461. */
 int bbx_matmul_f32(const float* a, const float* b, float* c, int m, int n, int k, long long lda,
@@ -259,8 +261,8 @@ int bbx_stream_plan_bulk(const bbx_stream_plan_t* plan);
 /* einsum contraction of the reference's "cutensor" plugin
  * (libraries/cutensor/contraction.h:25-63 params, :131-202 semantics):
  * out = alpha * sum lhs * rhs over modes absent from the output. Tensors are
- * COLUMN-major with int64 dims (cu.h:65-169). precision = BBX_F32 (SIMT) or
- * BBX_BF16 (tensor cores, f32 accumulate). */
+ * COLUMN-major with int64 dims (cu.h:65-169). precision = BBX_F32 (FP32
+ * accuracy) or BBX_BF16 (operands rounded to bf16, f32 accumulate). */
 int bbx_contraction(const float* lhs, int rank_l, const long long* dims_l, const int* modes_l,
                     const float* rhs, int rank_r, const long long* dims_r, const int* modes_r,
                     float* out, int rank_o, const int* modes_o, float alpha, int precision,
