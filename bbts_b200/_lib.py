@@ -36,6 +36,7 @@ SIGNATURES = {
     "bbx_check_device_status": (i32, [vp, C.POINTER(C.c_uint32)]),
     "bbx_matmul_f32": (i32, [pf, pf, pf, i32, i32, i32, i64, i64, i64, i32, i32, f32, f32, pf, i32,
                              i32, i64, i64, i64, vp]),
+    "bbx_matmul_f32_route": (i32, [i32, i32, i32, i32]),
     "bbx_matmul_tc": (i32, [i32, C.POINTER(TcProblem), i32, i32, vp]),
     "bbx_tc_plan_create": (i32, [i32, C.POINTER(TcProblem), i32, i32, C.POINTER(vp)]),
     "bbx_tc_plan_launch": (i32, [vp, vp]),

@@ -542,6 +542,8 @@ int bbx_matmul_f32(const float* a, const float* b, float* c, int m, int n, int k
   return BBX_OK;
 }
 
+int bbx_matmul_f32_route(int m, int n, int k, int batch) { return f3_wanted(m, n, k, batch) ? 1 : 0; }
+
 }  // extern "C"
 
 namespace bbx {

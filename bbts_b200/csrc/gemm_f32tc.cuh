@@ -39,11 +39,13 @@
 //
 // A problem whose operands could leave the range of the scheme (non-finite, or
 // large enough that a partial sum could overflow where an FP32 FMA chain does
-// not; see f3_in_range) is computed by the epilogue threads with FP32 FMAs in K
-// order, as k_gemm_f32 does.
+// not; see f3_in_range) is skipped by every warp's main loop and computed after
+// it by the epilogue warps, with FP32 FMAs in K order and k_gemm_f32_v's tiling
+// (f3_plain_tiles). No bounded wait spans that: the tensor-core part is over.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include "gemm_f32.cuh"
 #include "ptx.cuh"
 #include "tile_order.h"
 
@@ -139,7 +141,7 @@ __device__ __forceinline__ __nv_bfloat16 f3_bf16_finite(float x) {
   return fabsf(__bfloat162float(p)) <= 3.3895314e38f ? p : __ushort_as_bfloat16((unsigned short)(__float_as_uint(x) >> 16));
 }
 
-// The planes of any f32 value: f3_join gives the value back exactly (a NaN as a NaN).
+// The planes of any f32 value: f3_join2 gives the value back exactly (a NaN as a NaN).
 __device__ __forceinline__ void f3_split1(float x, __nv_bfloat16& p0, __nv_bfloat16& p1, __nv_bfloat16& p2) {
   const uint32_t mag = __float_as_uint(x) & 0x7FFFFFFFu;
   if (mag >= 0x7F800000u) {
@@ -153,10 +155,13 @@ __device__ __forceinline__ void f3_split1(float x, __nv_bfloat16& p0, __nv_bfloa
   p2 = __float2bfloat16_rn(__fmul_rn(__fsub_rn(r1, __bfloat162float(p1)), 256.f));
 }
 
-__device__ __forceinline__ float f3_join(const __nv_bfloat16* p, long long plane) {
-  const float lo = __fadd_rn(__fmul_rn(__bfloat162float(p[plane]), 1.f / 256.f),
-                             __fmul_rn(__bfloat162float(p[2 * plane]), 1.f / 65536.f));
-  return __fadd_rn(__bfloat162float(p[0]), lo);
+// Two neighbouring elements from the words that hold their planes.
+__device__ __forceinline__ float2 f3_join2(uint32_t p0, uint32_t p1, uint32_t p2) {
+  auto join = [](uint32_t a, uint32_t b, uint32_t c) {  // bf16 values in the upper halves
+    const float lo = __fadd_rn(__fmul_rn(__uint_as_float(b), 1.f / 256.f), __fmul_rn(__uint_as_float(c), 1.f / 65536.f));
+    return __fadd_rn(__uint_as_float(a), lo);
+  };
+  return make_float2(join(p0 << 16, p1 << 16, p2 << 16), join(p0 & 0xFFFF0000u, p1 & 0xFFFF0000u, p2 & 0xFFFF0000u));
 }
 
 // The planes of eight elements as 16-byte pieces, and the maximum of their magnitudes.
@@ -439,33 +444,130 @@ __device__ __forceinline__ float f3_finish(const F3Out& o, float acc, const floa
   return v;
 }
 
-// The FP32 form of one thread's row of the tile: columns [col0, col0 + ncols),
-// one FMA chain over k per output (k_gemm_f32's order).
-__device__ __noinline__ void f3_plain_row(const F3Args& args, int p, int batch, int row, int col0, int ncols) {
-  const F3Fields f = f3_fields(args, p);
-  const F3Out o = f3_out(args, p, batch);
-  if (row >= o.m || col0 >= o.n) return;
-  const __nv_bfloat16* __restrict__ A = f.a + batch * f.a_batch + row * f.a_row;
-  const __nv_bfloat16* __restrict__ B = f.b + batch * f.b_batch;
-  const long long ak = f.a_k, bk = f.b_k, bc = f.b_col, ap = f.a_plane, bpl = f.b_plane;
-  const int end = min(col0 + ncols, o.n);
-  for (int c0 = col0; c0 < end; c0 += 8) {
-    float s[8];
-    const __nv_bfloat16* bp[8];
+// The out-of-range problems' tiles of this CTA, by the 256 epilogue threads: 128 x 128
+// outputs at a time, 8 x 8 a thread in packed pairs, one FMA chain over k per output (the SIMT
+// kernels' order and bits). Operands come from the split planes, which join to the f32 values exactly and
+// have one layout for dense blocks and gathered tensors: a thread loads one aligned piece of eight
+// elements (three 16-byte loads) of A or B per eight steps of K, a step before it joins them into the
+// free one of two shared-memory buffers (the epilogue's, which no TMA writes).
+// Issue and barriers bound it, two warps a scheduler: 1024^3 with one infinity 162 us, 4096^3 4.3 ms;
+// k_gemm_f32_v, which reads f32, takes 105 us and 2.7 ms; one thread a row straight from the
+// planes took 7.7 ms for 1024^3. 16 steps a barrier (in the stages' memory): 4.4 ms. Joining at the
+// end of a step: 4.7.
+// Elements past the end of a row are masked: a row's padding in the planes may be unwritten.
+constexpr int kF3PlainBK = 8;
+constexpr int kF3PlainLd = 132;
+static_assert(2 * 2 * kF3PlainBK * kF3PlainLd * 4 <= kF3EpiWarps * kF3EpiSlot, "plain tiles' shared memory");
+static_assert(kF3EpiWarps == 8, "plain tiles take 256 threads");
+
+template <bool PAIR>
+__device__ __noinline__ void f3_plain_tiles(const F3Args& args, uint32_t stage_at, uint32_t meta_at, int unit, int units,
+                                            int rank) {
+  constexpr int BM = PAIR ? 256 : 128, BN = BM, BUF = kF3PlainBK * kF3PlainLd;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  float* const As = (float*)(smem_raw + stage_at);  // [2][BK][Ld]
+  float* const Bs = As + 2 * BUF;
+  const int4* const meta = (const int4*)(smem_raw + meta_at);
+  const int tid = threadIdx.x - 64, tx = tid & 15, ty = tid >> 4;
+  const bool of_b = tid >= 128;  // the operand that this thread loads
+  const int lt = tid & 127;
+  float* const put = of_b ? Bs : As;
+  auto sync = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+  sync();  // every warp is done with its part of that memory
+  for (int t0 = unit, rr = 0; t0 < args.total_tiles; t0 += units, ++rr) {
+    const F3Where w = f3_locate(meta, args.num_problems, snake_tile_of(t0, rr, args.total_tiles, unit, units));
+    if (w.k >= 0) continue;
+    const int k = -w.k;
+    const F3Fields f = f3_fields(args, w.p);
+    const F3Out o = f3_out(args, w.p, w.b);
+    const __nv_bfloat16* const src = of_b ? f.b + w.b * f.b_batch : f.a + w.b * f.a_batch;
+    const long long plane = of_b ? f.b_plane : f.a_plane;
+    const bool mn = (of_b ? f.b_mn : f.a_mn) != 0;
+    const long long pitch = of_b ? (mn ? f.b_k : f.b_col) : (mn ? f.a_k : f.a_row);
+    const int extent = of_b ? o.n : o.m;
+    const int m0 = w.tm * BM + rank * 128;
+    if (m0 >= o.m) continue;
+    for (int n0 = w.tn * BN; n0 < min(w.tn * BN + BN, o.n); n0 += 128) {
+      const int e0 = of_b ? n0 : m0;
+      // K-major: steps k0 .. k0 + 7 of row e0 + lt; MN-major: step k0 + lt / 16 of elements e0 + 8 (lt % 16) .. + 7
+      const int row0 = mn ? lt >> 4 : e0 + lt, col0 = mn ? e0 + 8 * (lt & 15) : 0;
+      // a piece has min(8, left) elements; left counts down along K where the steps do
+      const __nv_bfloat16* p = src + row0 * pitch + col0;
+      const long long step = mn ? kF3PlainBK * pitch : kF3PlainBK;
+      int left = mn ? extent - col0 : e0 + lt < extent ? k : 0;
+      int rows = mn ? k - row0 : 1;  // MN-major: steps left
+      uint4 q[3];
+      int have;
+      auto load = [&]() {
+        have = rows > 0 ? left : 0;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      s[u] = 0.f;
-      bp[u] = B + (long long)min(c0 + u, o.n - 1) * bc;
-    }
-    for (int k = 0; k < f.k; ++k) {
-      const float av = f3_join(A + k * ak, ap);
+        for (int i = 0; i < 3; ++i) q[i] = have > 0 ? __ldg((const uint4*)(p + i * plane)) : make_uint4(0u, 0u, 0u, 0u);
+        p += step;
+        if (mn) rows -= kF3PlainBK; else left -= kF3PlainBK;
+      };
+      auto store = [&](int buf) {
+        float v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) s[u] = fmaf(av, f3_join(bp[u] + k * bk, bpl), s[u]);
-    }
-    for (int u = 0; u < 8 && c0 + u < end; ++u) {
-      const int col = c0 + u;
-      float* cp = o.c + (o.c_col ? row + col * o.ldc : row * o.ldc + col);
-      *cp = f3_finish(o, s[u], cp, col);
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t *x = &q[0].x, *y = &q[1].x, *z = &q[2].x;
+          const float2 g = f3_join2(x[i], y[i], z[i]);
+          v[2 * i] = g.x;
+          v[2 * i + 1] = g.y;
+        }
+        if (have < 8) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = i < have ? v[i] : 0.f;
+        }
+        float* const b = put + buf * BUF;
+        if (mn) {
+          float* const r = b + (lt >> 4) * kF3PlainLd + 8 * (lt & 15);
+          *(float4*)r = make_float4(v[0], v[1], v[2], v[3]);
+          *(float4*)(r + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) b[i * kF3PlainLd + lt] = v[i];
+        }
+      };
+      f32pair acc[8][4];  // columns 2 j and 2 j + 1
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+      load();
+      store(0);
+      load();  // past the end: zeros
+      sync();
+      for (int k0 = 0, buf = 0; k0 < k; k0 += kF3PlainBK, buf ^= 1) {
+        store(buf ^ 1);  // read last before the barrier that ended the step before
+        load();
+        const float *a = As + buf * BUF + 4 * ty, *b = Bs + buf * BUF + 4 * tx;
+#pragma unroll
+        for (int kk = 0; kk < kF3PlainBK; ++kk) {
+          const float4 a0 = *(const float4*)(a + kk * kF3PlainLd), a1 = *(const float4*)(a + kk * kF3PlainLd + 64);
+          const ulonglong2 b0 = *(const ulonglong2*)(b + kk * kF3PlainLd), b1 = *(const ulonglong2*)(b + kk * kF3PlainLd + 64);
+          const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+          const f32pair bv[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const f32pair ai = pair_of(av[i]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fma_pair(acc[i][j], ai, bv[j]);
+          }
+        }
+        sync();
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int row = m0 + 4 * ty + (i & 3) + 64 * (i >> 2);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int col = n0 + 4 * tx + (j & 3) + 64 * (j >> 2);
+          if (row >= o.m || col >= o.n) continue;
+          float* const cp = o.c + (o.c_col ? row + col * o.ldc : row * o.ldc + col);
+          const float2 v = unpack_pair(acc[i][j >> 1]);
+          *cp = f3_finish(o, j & 1 ? v.y : v.x, cp, col);
+        }
+      }
     }
   }
 }
@@ -603,6 +705,7 @@ __device__ __forceinline__ void f3_gemm_body(const F3Args& args) {
   }
   griddep_launch();
   griddep_wait();  // the maxima below are the split's
+  int plain = 0;   // a problem is out of range
   if (warp >= 2) {
     // one warp per problem: its tiles, and whether its operands are in range
     for (int p = warp - 2; p < args.num_problems; p += kF3EpiWarps) {
@@ -616,11 +719,13 @@ __device__ __forceinline__ void f3_gemm_body(const F3Args& args) {
       }
       ma = __reduce_max_sync(0xffffffffu, ma);
       mb = __reduce_max_sync(0xffffffffu, mb);
-      if (lane == 0) meta[p] = make_int4(f.tile_start, f.tiles_m, f.tiles_n, f3_in_range(ma, mb, k) ? k : -k);
+      const bool in_range = f3_in_range(ma, mb, k);
+      plain |= !in_range;
+      if (lane == 0) meta[p] = make_int4(f.tile_start, f.tiles_m, f.tiles_n, in_range ? k : -k);
     }
   }
   tc_fence_before();
-  __syncthreads();
+  plain = __syncthreads_or(plain);
   if constexpr (PAIR) {
     __syncwarp();
     cluster_sync();
@@ -765,11 +870,8 @@ __device__ __forceinline__ void f3_gemm_body(const F3Args& args) {
     bool ok = true;
     for (int t0 = unit, rr = 0; t0 < args.total_tiles && ok; t0 += units, ++rr) {
       const F3Where w = locate(t0, rr);
+      if (w.k <= 0) continue;
       const int row0 = w.tm * BM + (int)rank * 128 + 32 * quarter, col0 = w.tn * BN + half * NC;
-      if (w.k <= 0) {
-        f3_plain_row(args, w.p, w.b, row0 + lane, col0, NC);
-        continue;
-      }
       const F3Out o = f3_out(args, w.p, w.b);
       float acc[NC];
 #pragma unroll
@@ -802,6 +904,9 @@ __device__ __forceinline__ void f3_gemm_body(const F3Args& args) {
       if (!ok) break;
       f3_store<NC>(o, row0, col0, lane, stage, acc);
     }
+    // all eight warps, whatever their waits came to
+    if (plain)
+      f3_plain_tiles<PAIR>(args, (uint32_t)((uint8_t*)epi - smem_raw), (uint32_t)((uint8_t*)meta - smem_raw), unit, units, (int)rank);
   }
 
   // in a pair the leader's MMAs read the peer's shared memory: neither CTA may

@@ -101,6 +101,9 @@ int bbx_matmul_f32(const float* a, const float* b, float* c, int m, int n, int k
                    long long ldb, long long ldc, int trans_a, int trans_b, float alpha, float beta,
                    const float* bias, int relu, int batch, long long stride_a, long long stride_b,
                    long long stride_c, void* stream);
+/* 1 when the size rule gives an m x n x k product (each of `batch`) to the tensor
+ * cores, 0 when to the SIMT kernel. Needs no device. */
+int bbx_matmul_f32_route(int m, int n, int k, int batch);
 
 /* One tensor-core block product. a/b are bf16 or e4m3 (row-major, pitches in
  * elements, pitch*elem_size and base pointers 16-byte aligned), c is f32 or
