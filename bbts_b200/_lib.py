@@ -34,6 +34,7 @@ SIGNATURES = {
     "bbx_last_error": (i32, [C.c_char_p, sz]),
     "bbx_num_sms": (i32, []),
     "bbx_check_device_status": (i32, [vp, C.POINTER(C.c_uint32)]),
+    "bbx_trim_scratch": (i32, []),
     "bbx_matmul_f32": (i32, [pf, pf, pf, i32, i32, i32, i64, i64, i64, i32, i32, f32, f32, pf, i32,
                              i32, i64, i64, i64, vp]),
     "bbx_matmul_f32_route": (i32, [i32, i32, i32, i32]),

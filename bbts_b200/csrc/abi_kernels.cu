@@ -473,6 +473,11 @@ int bbx_num_sms(void) {
   return d->sms;
 }
 
+int bbx_trim_scratch(void) {
+  scratch_trim();
+  return BBX_OK;
+}
+
 int bbx_check_device_status(void* stream, uint32_t* code_out) {
   DeviceState* d;
   int rc = device_state(&d);

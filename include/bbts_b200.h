@@ -90,6 +90,11 @@ int bbx_num_sms(void);
  * by kernels whose bounded waits ran out. Returns 0 or BBX_ERR_DEVICE. */
 int bbx_check_device_status(void* stream, uint32_t* code_out);
 
+/* Gives back the device memory that the library's scratch pool keeps between calls
+ * (512 MiB at most) and that no queued work uses. A caller whose other allocator runs
+ * out calls it, after a synchronisation. */
+int bbx_trim_scratch(void);
+
 /* ------------------------------------------------------------------ block matmul */
 /* FP32 matmul: C = alpha*op(A)*op(B) + beta*C (+bias[col]) (relu), batched
  * over `batch` with element strides. Large products run on the tensor cores (each
