@@ -64,8 +64,9 @@ static DeviceState g_dev[64];
 // Scratch kept by the pool across synchronisations. The device's default pool
 // keeps none: a call after a synchronisation then maps its scratch again, which
 // took 3-4 ms (a 201 x 160 x 130 contraction 4.0 ms alone against 0.15 ms among others).
-// 512 MiB holds the operand planes of an 8192^2 by 8192 x 2048 f32 product; the
-// runtime takes it back (scratch_trim) before it reports the device out of memory.
+// 512 MiB holds the operand planes of an 8192^2 by 8192 x 2048 f32 product; every
+// allocation of the library takes it back (scratch_reclaim) before it fails, and
+// bbx_trim_scratch does for other allocators.
 constexpr uint64_t kScratchKeep = 512ull << 20;
 
 template <int BN, bool AMN, bool BMN, bool FP8, bool EP8 = false>
@@ -207,6 +208,34 @@ void scratch_trim() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
   std::lock_guard<std::mutex> lk(g_dev_mu);
   if (g_dev[dev].scratch) cudaMemPoolTrimTo(g_dev[dev].scratch, 0);
+}
+
+void scratch_reclaim() {
+  // relaxed: another thread may be capturing, which this wait does not touch
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+  scratch_trim();
+  cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
+unsigned& failed_allocs() {
+  static thread_local unsigned n = 0;
+  return n;
+}
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    scratch_reclaim();
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (e == cudaErrorMemoryAllocation) ++failed_allocs();
+  }
+  return e;
 }
 
 static inline int grid_for(long long work_items, int threads, int sms) {
@@ -673,7 +702,7 @@ static int tc_plan_create(int in_dtype, const bbx_tc_problem_t* problems, int co
   }
   p->ep8 = max_k <= (in_dtype == BBX_E4M3 ? kTcFp8Ep8MaxK : tile_n == 512 && f32_c ? kTc2Ep8MaxK : kTcEp8MaxK);
   if (count > kTcMaxInline) {
-    cudaError_t e = cudaMalloc(&p->d_table, sizeof(TcProblem) * count);
+    cudaError_t e = device_alloc((void**)&p->d_table, sizeof(TcProblem) * count);
     if (e != cudaSuccess) { delete p; return set_error(BBX_ERR_CUDA, "cudaMalloc(plan table): %s", cudaGetErrorString(e)); }
     e = cudaMemcpy(p->d_table, p->host.data(), sizeof(TcProblem) * count, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { cudaFree(p->d_table); delete p; return set_error(BBX_ERR_CUDA, "plan upload: %s", cudaGetErrorString(e)); }
@@ -1073,7 +1102,7 @@ int bbx_stream_plan_create_kernel(const bbx_stream_op_t* ops, int count, int ker
   p->count = count;
   p->total_chunks = total;
   p->bulk = bulk;
-  cudaError_t e = cudaMalloc(&p->d_table, sizeof(StreamOp) * count);
+  cudaError_t e = device_alloc((void**)&p->d_table, sizeof(StreamOp) * count);
   if (e == cudaSuccess) e = cudaMemcpy(p->d_table, table.data(), sizeof(StreamOp) * count, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     if (p->d_table) cudaFree(p->d_table);

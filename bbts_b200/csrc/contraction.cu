@@ -747,7 +747,7 @@ int gather_plan_create(const GatherRec* recs, int count, GatherPlan** out, bool 
   p->total = chunks;
   p->bulk = bulk;
   p->wide = wide && !bulk;
-  cudaError_t e = cudaMalloc(&p->d, sizeof(GatherRec) * count);
+  cudaError_t e = device_alloc((void**)&p->d, sizeof(GatherRec) * count);
   if (e == cudaSuccess) e = cudaMemcpy(p->d, h.data(), sizeof(GatherRec) * count, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     if (p->d) cudaFree(p->d);

@@ -345,9 +345,9 @@ int f3_plan_create(const F3Mat* mats, int n_mats, const F3Spec* specs, int n_spe
     }
     p->parts.push_back({first, count, (int)tiles, (int)shape});
   }
-  cudaError_t e = cudaMalloc(&p->d_problems, sizeof(F3Problem) * n_specs);
+  cudaError_t e = device_alloc((void**)&p->d_problems, sizeof(F3Problem) * n_specs);
   if (e == cudaSuccess) e = cudaMemcpy(p->d_problems, probs.data(), sizeof(F3Problem) * n_specs, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&p->d_splits, sizeof(F3Split) * splits.size());
+  if (e == cudaSuccess) e = device_alloc((void**)&p->d_splits, sizeof(F3Split) * splits.size());
   if (e == cudaSuccess) e = cudaMemcpy(p->d_splits, splits.data(), sizeof(F3Split) * splits.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return set_error(BBX_ERR_CUDA, "f32 plan upload: %s", cudaGetErrorString(e));
   *out = p.release();

@@ -5,6 +5,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <vector>
+#include <cuda_runtime_api.h>
 #include "contraction.h"
 
 namespace bbx {
@@ -89,11 +90,20 @@ int f32_simt_plan_launch(F32SimtPlan* p, void* stream);
 void f32_simt_plan_destroy(F32SimtPlan* p);
 
 // Stream-ordered scratch from the library's pool (per device). The pool keeps
-// at most kScratchKeep bytes across synchronisations; scratch_trim gives
-// the unused part back.
-void* scratch_alloc(size_t bytes, void* stream);  // nullptr when the device is out of memory
+// at most kScratchKeep bytes across synchronisations. nullptr when the device is
+// out of memory.
+void* scratch_alloc(size_t bytes, void* stream);
 void scratch_free(void* p, void* stream);
+// Gives back what the pool holds and nothing uses; reclaim first waits for the device, so
+// that blocks whose release is still queued are among it. Before any allocation of the library's is
+// reported as failed; not by a thread that captures a stream.
 void scratch_trim();
+void scratch_reclaim();
+
+// cudaMalloc, once more after scratch_reclaim when the device is out of memory; what still fails
+// counts in failed_allocs (of the calling thread). No error stays behind for a launch check.
+cudaError_t device_alloc(void** p, size_t bytes);
+unsigned& failed_allocs();
 
 // 3-D bf16 tensor map: dims (cols, rows, planes), 128-byte swizzle (abi_kernels.cu).
 int make_map3(void* map, const void* base, long long cols, long long rows, long long z, long long pitch,

@@ -54,6 +54,7 @@ namespace bbts {
 namespace {
 
 void dag_cuda(cudaError_t e, const char* what) {
+  if (e == cudaErrorMemoryAllocation) ++bbx::failed_allocs();
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 void dag_bbx(int rc) {
@@ -401,9 +402,9 @@ void lower_for_tc(const std::vector<tensor_meta_t>& in_metas, const command_t& c
 }  // namespace
 
 // f32_tc: lower f32 products to the tensor cores, whose operand planes live in the
-// arena; *no_room is set when an arena with them does not fit the device.
-static dag_t* dag_build_as(runtime_t* rt, int policy, int tile_n, bool f32_tc, bool* no_room) {
-  auto d = std::make_unique<dag_t>();
+// arena; *planes: some are.
+static dag_t* dag_build_as(runtime_t* rt, int policy, int tile_n, bool f32_tc, bool* planes) {
+  std::unique_ptr<dag_t, void (*)(dag_t*)> d(new dag_t(), dag_destroy);  // a failed build keeps no device memory
   d->rt = rt;
   const tensor_factory_t& tf = *rt->tf;
 
@@ -574,10 +575,9 @@ static dag_t* dag_build_as(runtime_t* rt, int policy, int tile_n, bool f32_tc, b
   };
   // planes of a wave's f32 operands: a block is split once per wave, whatever products read it
   std::map<std::pair<int, tid_t>, tid_t> f3_stage;
-  bool any_f3 = false;
   for (int i = 0; i < N; ++i) {
     node_t& n = nodes[i];
-    any_f3 = any_f3 || n.f3;
+    *planes = *planes || n.f3;
     if (n.f3 && n.kind == NK_SIMT) {
       for (tid_t t : n.ins) {
         const auto key = std::make_pair(n.wave, t);
@@ -647,27 +647,14 @@ static dag_t* dag_build_as(runtime_t* rt, int policy, int tile_n, bool f32_tc, b
     offsets[tid] = off;
     arena = std::max(arena, off + bytes);
   }
-  if (arena) {
-    cudaError_t e = cudaMalloc(&d->arena, arena);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      bbx::scratch_trim();
-      e = cudaMalloc(&d->arena, arena);
-    }
-    if (e == cudaErrorMemoryAllocation && no_room && any_f3) {
-      cudaGetLastError();
-      *no_room = true;
-      return nullptr;
-    }
-    dag_cuda(e, "cudaMalloc(DAG arena)");
-  }
+  if (arena) dag_cuda(bbx::device_alloc(&d->arena, arena), "cudaMalloc(DAG arena)");
   d->arena_bytes = arena;
   for (auto& kv : offsets) d->tensors[kv.first].payload = (char*)d->arena + kv.second;
   for (auto& kv : d->tensors) {
     auto& tp = kv.second;
     if (tp.external || tp.deleted) continue;
     void* p = nullptr;
-    if (tp.bytes) dag_cuda(cudaMalloc(&p, tp.bytes), "cudaMalloc(DAG result)");
+    if (tp.bytes) dag_cuda(bbx::device_alloc(&p, tp.bytes), "cudaMalloc(DAG result)");
     tp.payload = p;
     d->persistent.push_back(p);
   }
@@ -1084,7 +1071,6 @@ static dag_t* dag_build_as(runtime_t* rt, int policy, int tile_n, bool f32_tc, b
     cudaStreamDestroy(origin);
     cudaStreamDestroy(s_mem);
     cudaStreamDestroy(s_tc);
-    dag_destroy(d.release());
     throw;
   }
   for (auto& e : ev) cudaEventDestroy(e);
@@ -1096,9 +1082,16 @@ static dag_t* dag_build_as(runtime_t* rt, int policy, int tile_n, bool f32_tc, b
 }
 
 dag_t* dag_build(runtime_t* rt, int policy, int tile_n) {
-  bool no_room = false;
-  dag_t* d = dag_build_as(rt, policy, tile_n, true, &no_room);
-  return no_room ? dag_build_as(rt, policy, tile_n, false, nullptr) : d;
+  // Where the planes leave no room, for themselves or for a result or a table after
+  // them, the SIMT groups, which need none.
+  const unsigned failed = bbx::failed_allocs();
+  bool planes = false;
+  try {
+    return dag_build_as(rt, policy, tile_n, true, &planes);
+  } catch (...) {
+    if (!planes || bbx::failed_allocs() == failed) throw;
+  }
+  return dag_build_as(rt, policy, tile_n, false, &planes);
 }
 
 void dag_launch(dag_t* d, cudaStream_t st) { dag_cuda(cudaGraphLaunch(d->exec, st), "cudaGraphLaunch"); }

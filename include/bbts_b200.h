@@ -91,8 +91,9 @@ int bbx_num_sms(void);
 int bbx_check_device_status(void* stream, uint32_t* code_out);
 
 /* Gives back the device memory that the library's scratch pool keeps between calls
- * (512 MiB at most) and that no queued work uses. A caller whose other allocator runs
- * out calls it, after a synchronisation. */
+ * (512 MiB at most) and that no queued work uses. The library's own allocations do this
+ * before they fail; a caller whose other allocator runs out calls it, after a
+ * synchronisation. */
 int bbx_trim_scratch(void);
 
 /* ------------------------------------------------------------------ block matmul */

@@ -1,5 +1,5 @@
 """FP32 products take scratch that the SIMT kernels did not: on a device that is nearly full,
-what fitted without it still runs."""
+what fitted without it still runs. The device is filled from the host, but for a stated rest."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -15,6 +15,63 @@ def T(cuda):
     from bbts_b200 import lib, ops, runtime
     assert lib.bbx_matmul_f32_route(N, N, N, 1) == 1
     return torch, ops, runtime, lib
+
+
+class _Filled:
+    """All device memory but `rest` bytes taken (in whole 2 MiB pieces)."""
+
+    def __init__(self, torch, lib, rest):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        lib.bbx_trim_scratch()
+        free = torch.cuda.mem_get_info()[0]
+        assert free > rest
+        self.torch = torch
+        self.block = torch.empty((free - rest) >> 21 << 21, dtype=torch.uint8, device="cuda")
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.torch.cuda.synchronize()
+        self.block = None
+        self.torch.cuda.empty_cache()
+
+
+def _simt(torch, ops, a, b):
+    c = torch.empty(N, N, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):  # a captured call runs the SIMT kernel
+        ops.matmul_f32(a, b, c)
+    graph.replay()
+    torch.cuda.synchronize()
+    return c
+
+
+# nine operands' planes (864 MiB) and eight results (512): everything fits; the arena fits but not the results after
+# it; not even the arena
+@pytest.mark.parametrize("rest,planes", [(2 << 30, True), (1100 << 20, False), (700 << 20, False)])
+def test_compiled_list_without_room_for_planes(T, rest, planes):
+    torch, ops, runtime, lib = T
+    rt = runtime.Runtime()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = [torch.randn(N, N, device="cuda", generator=g) for _ in range(9)]
+    for t, v in enumerate(x):
+        rt.put_dense(t, v.cpu().numpy())
+    mm = rt.impl("matrix_mult", ["dense"] * 2, ["dense"])
+    for j in range(8):
+        rt.apply(mm, [0, 1 + j], [100 + j])
+    simt, got = _simt(torch, ops, x[0], x[8]), torch.empty(N, N, device="cuda")
+    tc = torch.empty(N, N, device="cuda")
+    ops.matmul_f32(x[0], x[8], tc)
+    with _Filled(torch, lib, rest):
+        dag = rt.build_dag()
+        dag.launch()
+        dag.fetch(107, got.data_ptr(), BLOCK, on_device=True)
+    assert torch.equal(got, tc if planes else simt)
+    dag.close()
+    rt.close()
 
 
 def test_other_allocators_get_the_scratch_back(T):
