@@ -185,12 +185,23 @@ int device_status_and_sms(uint32_t** status, int* sms) {
   return BBX_OK;
 }
 
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 // The pool is thread-safe and orders a block's reuse by stream.
-void* scratch_alloc(size_t bytes, void* stream) {
+void* scratch_alloc(size_t bytes, void* stream, bool must) {
   DeviceState* d;
   if (device_state(&d)) return nullptr;
   void* p = nullptr;
-  const cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, d->scratch, (cudaStream_t)stream);
+  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, d->scratch, (cudaStream_t)stream);
+  if (e == cudaErrorMemoryAllocation && must) {
+    cudaGetLastError();
+    scratch_reclaim();
+    e = cudaMallocFromPoolAsync(&p, bytes, d->scratch, (cudaStream_t)stream);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();  // a failed allocation must not show up at the next launch check
     set_error(BBX_ERR_CUDA, "scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
@@ -545,9 +556,7 @@ int bbx_matmul_f32(const float* a, const float* b, float* c, int m, int n, int k
   // planes the SIMT kernel, which needs none, runs. A fused ReLU marks a
   // pre-activation (FmaChain).
   if (!relu && !FmaChain::active() && f3_wanted(m, n, k, batch)) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    BBX_CUDA(cudaStreamIsCapturing(st, &cap));
-    if (cap == cudaStreamCaptureStatusNone) {
+    if (!capturing(st)) {
       F3Mat mats[2] = {trans_a ? f3_dense(a, k, m, lda, batch, stride_a, true) : f3_dense(a, m, k, lda, batch, stride_a, false),
                        trans_b ? f3_dense(b, n, k, ldb, batch, stride_b, false) : f3_dense(b, k, n, ldb, batch, stride_b, true)};
       const size_t ba = f3_mat_bytes(mats[0]), bb = f3_mat_bytes(mats[1]);
@@ -892,7 +901,7 @@ int bbx_quantize_e4m3(int src_dtype, const void* in, void* out, int rows, int co
   cudaStream_t st = (cudaStream_t)stream;
   // the absmax word is stream-ordered scratch of this call, so quantisations
   // on different streams never share it
-  unsigned int* amax = (unsigned int*)scratch_alloc(4, st);
+  unsigned int* amax = (unsigned int*)scratch_alloc(4, st, !capturing(st));
   if (!amax) return BBX_ERR_CUDA;
   BBX_CUDA(cudaMemsetAsync(amax, 0, 4, st));
   uint8_t* o = (uint8_t*)out;
@@ -922,7 +931,7 @@ int bbx_quantize_e4m3_batched(int src_dtype, const void* const* in, void* const*
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   // one absmax word per block, stream-ordered scratch of this call
-  unsigned int* amax = (unsigned int*)scratch_alloc(sizeof(unsigned int) * count, st);
+  unsigned int* amax = (unsigned int*)scratch_alloc(sizeof(unsigned int) * count, st, !capturing(st));
   if (!amax) return BBX_ERR_CUDA;
   BBX_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned int) * count, st));
   cudaError_t le = src_dtype == BBX_F32

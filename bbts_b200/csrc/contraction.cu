@@ -826,7 +826,7 @@ extern "C" int bbx_contraction(const float* lhs, int rank_l, const long long* di
     }
     lbytes = (size_t)(L.lc_elems * esz + 16);
     rbytes = (size_t)(L.rc_elems * esz + 16);
-    ws = (char*)scratch_alloc(up(lbytes) + up(rbytes) + cbytes, stream);
+    ws = (char*)scratch_alloc(up(lbytes) + up(rbytes) + cbytes, stream, !capturing(st));
     if (!ws) return BBX_ERR_CUDA;
   }
   void *Lc = ws, *Rc = ws + up(lbytes);

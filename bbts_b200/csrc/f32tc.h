@@ -91,8 +91,9 @@ void f32_simt_plan_destroy(F32SimtPlan* p);
 
 // Stream-ordered scratch from the library's pool (per device). The pool keeps
 // at most kScratchKeep bytes across synchronisations. nullptr when the device is
-// out of memory.
-void* scratch_alloc(size_t bytes, void* stream);
+// out of memory; with `must`, only after scratch_reclaim.
+void* scratch_alloc(size_t bytes, void* stream, bool must = false);
+bool capturing(cudaStream_t st);
 void scratch_free(void* p, void* stream);
 // Gives back what the pool holds and nothing uses; reclaim first waits for the device, so
 // that blocks whose release is still queued are among it. Before any allocation of the library's is

@@ -248,14 +248,15 @@ void block_storage_t::_make_room(size_t need, cudaStream_t st) {
   }
 }
 
-// A block from the storage's pool; when the device is out of memory, once more
-// after the library's scratch pool has given back what it keeps.
+// A block from the storage's pool; when the device is out of memory, once more after the
+// library's scratch pool has given back what it keeps, queued commands' scratch included.
 static void* pool_block(size_t bytes, cudaMemPool_t pool, cudaStream_t st, const char* what) {
   void* p = nullptr;
   cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, st);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    bbx::scratch_trim();
+    if (bbx::capturing(st)) bbx::scratch_trim();
+    else bbx::scratch_reclaim();
     e = cudaMallocFromPoolAsync(&p, bytes, pool, st);
   }
   cuda_ok(e, what);

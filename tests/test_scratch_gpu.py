@@ -74,6 +74,29 @@ def test_compiled_list_without_room_for_planes(T, rest, planes):
     rt.close()
 
 
+def test_commands_whose_scratch_is_still_queued(T):
+    """Products one after another, nothing waited for: a block's allocation that the queued products'
+    scratch stands in the way of waits for it."""
+    torch, ops, runtime, lib = T
+    rt = runtime.Runtime()
+    g = torch.Generator(device="cuda").manual_seed(2)
+    a, b = torch.randn(N, N, device="cuda", generator=g), torch.randn(N, N, device="cuda", generator=g)
+    rt.put_dense(0, a.cpu().numpy())
+    rt.put_dense(1, b.cpu().numpy())
+    mm = rt.impl("matrix_mult", ["dense"] * 2, ["dense"])
+    count = 8
+    for j in range(count):
+        rt.apply(mm, [0, 1], [100 + j])
+    simt = _simt(torch, ops, a, b)
+    with _Filled(torch, lib, count * BLOCK + PLANES):  # the blocks, and half of one product's scratch
+        rt.run()
+    ref = a.double() @ b.double()
+    for j in range(count):  # each on the tensor cores or, without room for its planes, on the SIMT kernel
+        got = torch.from_numpy(rt.get_dense(100 + j)).cuda()
+        assert torch.equal(got, simt) or ((got.double() - ref).norm() < 1e-6 * ref.norm())
+    rt.close()
+
+
 def test_other_allocators_get_the_scratch_back(T):
     torch, ops, runtime, lib = T
     a, b, c = (torch.randn(N, N, device="cuda") for _ in range(3))
