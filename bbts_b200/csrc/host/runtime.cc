@@ -8,7 +8,6 @@
 
 #include <algorithm>
 #include <cerrno>
-#include <chrono>
 #include <cstring>
 #include <cmath>
 #include <numeric>
@@ -632,6 +631,43 @@ std::unordered_set<command_id_t> pre_activations(const std::vector<command_ptr_t
   return found;
 }
 
+// Holds the device before a recorded command until the host has queued the whole command, so that
+// the events around it time the device alone: a host thread that another process keeps off its core
+// (6-30 ms seen), or that waits for memory to be mapped, left the device idle inside the bracket. One
+// thread polls a host word, 20 ms at most (a command that waits for the device itself, e.g. a spill
+// file's, is only held up that long). Commands over 300 us, none of which takes the device 60, in 150
+// recorded lists of 160: 3 with it, 35 in 96 without.
+__global__ void k_hold(const volatile unsigned* word, unsigned n) {
+  unsigned long long t0, t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+  do {
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  } while (*word < n && t - t0 < 20000000ull);
+}
+
+class device_hold_t {
+ public:
+  explicit device_hold_t(cudaStream_t st) : st_(st) {
+    cuda_ok(cudaHostAlloc(&word_, sizeof(unsigned), cudaHostAllocMapped), "cudaHostAlloc(hold)");
+    *word_ = 0;
+  }
+  ~device_hold_t() {
+    __atomic_store_n(word_, ~0u, __ATOMIC_RELEASE);
+    cudaStreamSynchronize(st_);  // the last hold has read the word
+    cudaFreeHost(word_);
+  }
+  void close(cudaStream_t st) {
+    k_hold<<<1, 1, 0, st>>>(word_, ++n_);
+    cuda_ok(cudaGetLastError(), "k_hold");
+  }
+  void open() { __atomic_store_n(word_, n_, __ATOMIC_RELEASE); }
+
+ private:
+  cudaStream_t st_;
+  unsigned* word_ = nullptr;
+  unsigned n_ = 0;
+};
+
 // Executes one APPLY / REDUCE on the runtime stream (the per-op path).
 void execute_command(runtime_t& rt, command_t& cmd, cudaStream_t st, bool keep_chain) {
   const bbx::FmaChain chain(keep_chain);
@@ -854,6 +890,7 @@ void runtime_t::run_per_op(int policy, std::vector<std::pair<op_features_t, floa
   int rr = 0;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> evs;
   std::vector<op_features_t> feats;
+  std::unique_ptr<device_hold_t> hold(record ? new device_hold_t(stream) : nullptr);
   while (true) {
     tid_t dead;
     while (rs.try_get_to_remove(&dead)) {
@@ -894,31 +931,17 @@ void runtime_t::run_per_op(int policy, std::vector<std::pair<op_features_t, floa
       feats.push_back(features(*cmd, &hint));
       cudaEventCreate(&e0);
       cudaEventCreate(&e1);
+      hold->close(s);
+      cudaEventRecord(e0, s);
     }
-    // A host thread held up between the two events (another process on its core,
-    // memory being mapped) leaves the device idle inside the bracket: a command
-    // that kept the host longer than any launch takes, and whose measured time is
-    // mostly that, is timed again. Commands are functions of their inputs, uniform aside.
-    for (int attempt = 0;; ++attempt) {
-      const auto h0 = std::chrono::steady_clock::now();
-      if (record) cudaEventRecord(e0, s);
-      storage->begin_command();
-      try {
-        execute_command(*this, *cmd, s, keep_chain.count(cmd->id) != 0);
-      } catch (...) {
-        storage->end_command(s);
-        throw;
-      }
+    storage->begin_command();
+    try {
+      execute_command(*this, *cmd, s, keep_chain.count(cmd->id) != 0);
+    } catch (...) {
       storage->end_command(s);
-      if (!record) break;
-      cudaEventRecord(e1, s);
-      const double host_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - h0).count();
-      if (host_us < 150.0 || attempt == 2 || cmd->get_num_inputs() == 0) break;
-      cuda_ok(cudaEventSynchronize(e1), "record sync");
-      float ms = 0;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (ms * 1000.f < 0.5 * host_us) break;  // the launch queue was full: the device was busy
+      throw;
     }
+    storage->end_command(s);
     if (hint_readers) {
       for (size_t j = 0; j < cmd->get_num_inputs(); ++j) {
         const tid_t t = cmd->get_input(j).tid;
@@ -930,7 +953,11 @@ void runtime_t::run_per_op(int policy, std::vector<std::pair<op_features_t, floa
         storage->set_readers_left(t, r == readers_left.end() ? 0 : r->second);
       }
     }
-    if (record) evs.push_back({e0, e1});
+    if (record) {
+      cudaEventRecord(e1, s);
+      hold->open();
+      evs.push_back({e0, e1});
+    }
     if (K > 1) {
       cudaEvent_t done = new_event();
       cuda_ok(cudaEventRecord(done, s), "record done");

@@ -386,7 +386,9 @@ int bbx_rt_run(bbx_rt_t* rt, int policy);
 int bbx_rt_set_workers(bbx_rt_t* rt, int workers);
 /* Same as bbx_rt_run on one stream, recording each command's (12 features,
  * latency in us, the ud's get_complexity_hint) as training data for the cost
- * model; any output pointer may be null; returns the record count in *n_out. */
+ * model; any output pointer may be null; returns the record count in *n_out.
+ * The device is held before each command until the host has queued it (20 ms at
+ * most), so the latencies are the device's own. */
 int bbx_rt_record(bbx_rt_t* rt, int policy, float* features, float* latency_us, double* hints, int cap,
                   int* n_out);
 

@@ -1,0 +1,62 @@
+"""Recorded timings: every command runs once, and the time is the device's."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def R(cuda):
+    from bbts_b200 import runtime
+    return runtime
+
+
+def test_each_command_runs_once(R):
+    """A long product whose blocks the pools have to map first (milliseconds of host time): recording the
+    list takes about what running it does, on a fresh runtime each, not a multiple."""
+    n = 16384
+
+    def wall(record):
+        rt = R.Runtime()
+        rt.put(0, R.dense_meta(rt.fmt("dense"), n, n))
+        rt.fill_philox(0, 0, 1, 0.0, 1.0)
+        rt.apply(rt.impl("matrix_mult", ["dense"] * 2, ["dense"]), [0, 0], [1])
+        t0 = time.perf_counter()
+        if record:
+            _, lat = rt.record()
+            assert len(lat) == 1 and lat[0] > 10e3
+        else:
+            rt.run()
+        t0 = time.perf_counter() - t0
+        rt.close()
+        return t0
+    wall(False)  # the process's first kernels
+    run, record = wall(False), wall(True)
+    assert record < 1.6 * run, (record, run)
+
+
+@pytest.mark.parametrize("spill", [False, True])
+def test_recorded_blocks_are_the_runs(R, spill, tmp_path):
+    """Also where commands wait for the device themselves (spilled blocks through a file)."""
+    got = []
+    for record in (False, True):
+        rt = R.Runtime()
+        rng = np.random.default_rng(3)
+        for t in range(6):
+            rt.put_dense(t, rng.standard_normal((256, 256)).astype(np.float32))
+        if spill:
+            rt.set_storage_budget(5 * 256 * 1024, host_bytes=256 * 1024, spill_file=str(tmp_path / ("f%d" % record)))
+        mm, add = rt.impl("matrix_mult", ["dense"] * 2, ["dense"]), rt.impl("matrix_add", ["dense"] * 2, ["dense"])
+        for j in range(6):
+            rt.apply(mm, [j, (j + 1) % 6], [10 + j])
+            rt.apply(add, [10 + j, j], [20 + j])
+        if record:
+            _, lat = rt.record()
+            assert len(lat) == 12 and (lat > 0).all()
+        else:
+            rt.run()
+        got.append([rt.get_dense(20 + j) for j in range(6)])
+        rt.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
