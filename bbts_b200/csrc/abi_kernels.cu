@@ -568,7 +568,7 @@ int bbx_matmul_f32(const float* a, const float* b, float* c, int m, int n, int k
         s.c = c; s.bias = bias;
         s.m = m; s.n = n; s.k = k;
         s.ldc = ldc; s.c_batch = stride_c;
-        s.alpha = alpha; s.beta = beta; s.relu = relu;
+        s.alpha = alpha; s.beta = beta;
         const int rc = f3_run(mats, s, stream);
         scratch_free(ws, stream);
         return rc;

@@ -187,7 +187,6 @@ int build_problem(const F3Mat* mats, const F3Spec& s, Shape shape, F3Problem* ou
   out->f.c_col = s.c_col ? 1 : 0;
   out->f.alpha = s.alpha;
   out->f.beta = s.beta;
-  out->f.relu = s.relu;
   return BBX_OK;
 }
 

@@ -21,7 +21,7 @@ struct F3Mat {
   void* ws = nullptr;  // f3_mat_bytes, 256-byte aligned
 };
 
-// C = alpha op(A) op(B) (+ beta C) (+ bias) (relu), batched. a, b: indices of the operands.
+// C = alpha op(A) op(B) (+ beta C) (+ bias), batched. a, b: indices of the operands.
 struct F3Spec {
   int a = 0, b = 0;
   float* c = nullptr;
@@ -30,7 +30,6 @@ struct F3Spec {
   long long ldc = 0, c_batch = 0;
   bool c_col = false;
   float alpha = 1.f, beta = 0.f;
-  int relu = 0;
 };
 
 // True when an m x n x k product (each of `batch`) runs on the tensor cores

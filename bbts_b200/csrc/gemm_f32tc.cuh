@@ -79,7 +79,6 @@ struct F3Fields {
   int a_mn, b_mn;              // operand tiles are MN-major
   int c_col;                   // element (i, j) of C at c[i + j * ldc], else c[i * ldc + j]
   float alpha, beta;
-  int relu;
 };
 struct alignas(64) F3Problem {
   CUtensorMap tmap_a, tmap_b;  // split planes, box 64 columns x 128 rows (K-major) or 64 x 64 (MN-major)
@@ -414,7 +413,7 @@ struct F3Out {
   float* c;          // of the tile's batch
   const float* bias;
   long long ldc;
-  int m, n, relu;
+  int m, n;
   float alpha, beta;
   bool plain, c_col;
 };
@@ -427,10 +426,9 @@ __device__ __forceinline__ F3Out f3_out(const F3Args& args, int p, int batch) {
   o.ldc = f.ldc;
   o.m = f.m;
   o.n = f.n;
-  o.relu = f.relu;
   o.alpha = f.alpha;
   o.beta = f.beta;
-  o.plain = f.beta == 0.f && !f.bias && !f.relu;
+  o.plain = f.beta == 0.f && !f.bias;
   o.c_col = f.c_col != 0;
   return o;
 }
@@ -440,7 +438,6 @@ __device__ __forceinline__ float f3_finish(const F3Out& o, float acc, const floa
   if (o.plain) return v;
   if (o.beta != 0.f) v += o.beta * *cp;
   if (o.bias) v += o.bias[col];
-  if (o.relu) v = v > 0.f ? v : 0.f;
   return v;
 }
 
@@ -575,7 +572,7 @@ __device__ __noinline__ void f3_plain_tiles(const F3Args& args, uint32_t stage_a
 // One warp's 32 rows x NC columns of C from its accumulators (lane l holds row
 // row0 + l). Row-major C goes through the warp's 32 x 16 buffer, so that each
 // store writes whole 64-byte row segments: 4 lanes x 16 bytes of 8 rows, or, where
-// C's rows are not 16-byte aligned (or there is a beta, a bias, a ReLU), 16 lanes of
+// C's rows are not 16-byte aligned (or there is a beta or a bias), 16 lanes of
 // 2 rows (4-byte stores of 8 rows each, every lane its own 16 bytes, made a lone
 // 501^3 product 27.6 us, now 25.0). Columns of a column-major C are already 32
 // consecutive elements across the lanes.
