@@ -25,8 +25,10 @@ bool FmaChain::active() { return t_fma_chain; }
 // tensor cores 1.15 us per 64 steps, after about 10 us more of launches (two
 // kernels, their prologues) and the operands' split (10 bytes moved per element at 4 TB/s):
 // 128 x 128 x 64 7 against 17 us, 256^3 29 against 28, 512^3 54 against 29, 4096^3 2700 against 750.
-// From K = 64 on its error is below the FMA chain's for every size measured
-// (normwise 0.8e-7 against 1.4e-7 at K = 64, 1.7e-7 against 11e-7 at K = 4096).
+// From K = 64 on its error is below the FMA chain's for every size measured, on normals and
+// on data of one sign (normwise 0.8e-7 against 1.4e-7 at K = 64, 1.7e-7 against 11e-7 at
+// K = 4096). Only short sums that one huge term dominates are summed better by the chain
+// (log-normals, sigma = 2, K <= 256: 3.7e-7 against 1.9e-7).
 bool f3_wanted(long long m, long long n, long long k, long long batch) {
   if (k < 64 || std::min(m, n) < 16 || batch <= 0 || batch > 65535) return false;
   const double tiles = (double)((m + 127) / 128) * ((n + 127) / 128) * batch;

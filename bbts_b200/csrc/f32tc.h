@@ -34,7 +34,9 @@ struct F3Spec {
 
 // True when an m x n x k product (each of `batch`) runs on the tensor cores
 // rather than on the SIMT kernels. The per-call and the grouped paths share
-// this rule, so both give the same bits.
+// this rule and give the same bits, except where there is no room for the planes
+// (per call: no scratch; a compiled list: built without them), and for a dense
+// product under stream capture: those run the SIMT kernels.
 bool f3_wanted(long long m, long long n, long long k, long long batch);
 
 // While one lives (with on = true), the f32 products that its thread enqueues keep the SIMT
@@ -42,6 +44,7 @@ bool f3_wanted(long long m, long long n, long long k, long long batch);
 // reaches a ReLU (directly or through adds): the sign of a pre-activation near 0
 // decides its mask, and a flipped mask moves a whole term of a gradient (1e-3 of its
 // norm from one flip in 10^6), so these masks stay those of the plain FP32 path, bit for bit.
+// Other ops between the product and the ReLU, and a ReLU in a later list, are not followed.
 class FmaChain {
  public:
   explicit FmaChain(bool on);

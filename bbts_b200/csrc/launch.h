@@ -1,7 +1,8 @@
 // Launch of a kernel that may start before its predecessor in the stream has
 // finished (programmatic dependent launch): the kernel runs griddep_wait (ptx.cuh)
 // before it touches memory. Its launch latency and prologue then overlap the
-// predecessor's tail. Behind anything but such a kernel it is a plain launch.
+// predecessor's tail. Behind anything but such a kernel it is a plain launch. The f32
+// SIMT products and the quantisation kernels have no such wait and launch plainly.
 #pragma once
 #include <cuda_runtime.h>
 #include <utility>

@@ -99,8 +99,10 @@ int bbx_trim_scratch(void);
 /* ------------------------------------------------------------------ block matmul */
 /* FP32 matmul: C = alpha*op(A)*op(B) + beta*C (+bias[col]) (relu), batched
  * over `batch` with element strides. Large products run on the tensor cores (each
- * operand split into three bf16 planes in stream-ordered scratch; FP32 accuracy),
- * small ones, and all under stream capture, on a SIMT kernel. Replaces dense_matrix_mult_t::mult
+ * operand split into three bf16 planes in stream-ordered scratch, 6 bytes an
+ * element; FP32 accuracy), small ones, all under stream capture and all whose
+ * scratch cannot be had on a SIMT kernel. The two round differently, so a call's bits
+ * can differ under capture or on a full device. Replaces dense_matrix_mult_t::mult
  * (dense_matrix_mult.cc:78-82: cblas_sgemm RowMajor with trans flags b0/b1) and
  * the batched cblas_sgemm_batch_strided of contraction.h:439-461. */
 int bbx_matmul_f32(const float* a, const float* b, float* c, int m, int n, int k, long long lda,
