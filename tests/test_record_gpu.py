@@ -33,7 +33,7 @@ def test_each_command_runs_once(R):
         rt.close()
         return t0
     wall(False)  # the process's first kernels
-    run, record = wall(False), wall(True)
+    run, record = (min(wall(r) for _ in range(3)) for r in (False, True))  # the least disturbed of three
     assert record < 1.6 * run, (record, run)
 
 

@@ -100,6 +100,7 @@ def test_commands_whose_scratch_is_still_queued(T):
 def test_other_allocators_get_the_scratch_back(T):
     torch, ops, runtime, lib = T
     a, b, c = (torch.randn(N, N, device="cuda") for _ in range(3))
+    ops.matmul_f32(a, b, c)  # loads the kernels
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     lib.bbx_trim_scratch()
